@@ -1704,6 +1704,11 @@ class CudaOps:
                            _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_float(scale),
                            _c_int(window or 0), _c_int(keep_first), _c_void_p(_ptr(sinks)))
             return out
+        if (q.dtype == torch.float32 and not window and sinks is None
+                and self.lib.mlxone_attention_f32_supports(_c_int(head_dim), _c_int(heads),
+                                                           _c_int(kv_heads))):
+            self._attention_f32(q, out, heads, kv_heads, head_dim, scale, ctx, view)
+            return out
         self._call("mlxone_attention_generic", _c_void_p(_ptr(q)), _c_void_p(_ptr(view.kv)),
                    _c_void_p(_ptr(view.block_table)), _c_int(width),
                    _c_int(view.page_size), _c_int(pages),
@@ -1712,6 +1717,35 @@ class CudaOps:
                    _c_int(head_dim), _c_float(scale), _c_int(window or 0),
                    _c_int(code), _c_void_p(_ptr(sinks)), _c_void_p(_ptr(self.error_flag)))
         return out
+
+    def _attention_f32(self, q, out, heads, kv_heads, head_dim, scale, ctx, view):
+        """The 32-bit engine's attention over every earlier key: single tokens and portions each
+        by a launch of their own, one block per unit of 64 keys where whole rows would be too few
+        blocks for two on every SM (one token of a request at position 140: 8 blocks or 24)."""
+        tokens, width = q.shape[0], view.block_table.shape[1]
+        if ctx.max_portion == 1 and tokens == ctx.requests:
+            singles = tokens
+        else:
+            singles = min(getattr(ctx, "leading_single", 0), ctx.requests)
+        units = -(-min(ctx.max_context, width * view.page_size) // 64)
+        group = heads // kv_heads
+        for first, end, single in ((0, singles, 1), (singles, tokens, 0)):
+            if first == end:
+                continue
+            tiles = end - first if single else -(-(end - first) // (32 // group))
+            values = (end - first) * heads * units * (head_dim + 4)
+            partial = None
+            if 1 < units <= 65535 and tiles * kv_heads < 2 * self._sm_count and values <= 1 << 26:
+                partial = torch.empty(values, dtype=torch.float32, device=self.device)
+            self._call("mlxone_attention_f32", _c_void_p(_ptr(q)), _c_void_p(_ptr(view.kv)),
+                       _c_void_p(_ptr(view.block_table)), _c_int(width), _c_int(view.page_size),
+                       _c_int(view.kv.shape[1]), _c_void_p(_ptr(ctx.positions)),
+                       _c_void_p(_ptr(ctx.token_request)), _c_void_p(_ptr(out)),
+                       _c_void_p(_ptr(partial)), _c_int(first), _c_int(end), _c_int(single),
+                       _c_int(0 if partial is None else units), _c_int(heads), _c_int(kv_heads),
+                       _c_int(head_dim), _c_float(scale), _c_void_p(_ptr(self.error_flag)))
+            if partial is not None:
+                self.launches += 1          # the merge kernel
 
     def _shaped_attention(self, q, heads, kv_heads, head_dim, scale, ctx, view, cap, slopes, least_slope):
         """paged_attention with capped or distance-biased scores, on the same kernels built with the

@@ -1,0 +1,75 @@
+"""The 32-bit engine's products and attention at the edges of their tiles, sections of K and units of
+keys, against 64 bits; and that a row's or a query's result is the same bits in every kernel."""
+
+import pytest
+import torch
+
+from test_gpu_kernels import make_batch, on_cpu, ops, plain  # noqa: F401  (fixtures)
+from mlx_one_b200.parts.base import PagedKeyValues, PagedView
+
+pytestmark = pytest.mark.gpu
+DEVICE = "cuda:0"
+
+
+@pytest.mark.parametrize("n,k", [(1, 8), (5, 7), (37, 520), (64, 512), (100, 1032), (50, 4608),
+                                 (33, 30), (2500, 136), (9500, 72)])
+def test_products_of_any_number_of_rows(ops, n, k):
+    """1 to 16 rows (the streaming kernel where K is a multiple of 8), then tiles of 32, 64 and 128
+    rows; rows that are a slice of wider ones, aligned or not."""
+    generator = torch.Generator(DEVICE).manual_seed(n * 10000 + k)
+    normal = lambda *shape: torch.randn(shape, generator=generator, device=DEVICE)
+    w, bias = normal(n, k), normal(n)
+    wide = normal(130, k + 9)
+    want = wide[:, 1:k + 1].double() @ w.double().T + bias.double()
+    # every value passes one chain of at most 32 FMAs and k / 256 + 10 additions
+    bound = (32 + k / 256 + 10) * 2.0 ** -24 * (wide[:, 1:k + 1].abs().double() @ w.abs().double().T +
+                                                bias.abs().double())
+    first = None
+    for m in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 130):
+        for a in (wide[:m, 1:k + 1], wide[:m, 1:k + 1].contiguous()):
+            got = ops.linear(a, w, bias)
+            assert ((got.double() - want[:m]).abs() <= bound[:m]).all(), (m, a.stride())
+            first = got[0] if first is None else first
+            assert torch.equal(got[0], first), (m, a.stride())
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [
+    (16, 8, 64, 16), (24, 8, 64, 16), (4, 4, 32, 4), (12, 1, 128, 32), (32, 1, 64, 64)])
+@pytest.mark.parametrize("portions,histories", [
+    ([1, 1, 1, 1, 1], [0, 62, 63, 64, 700]), ([1, 1, 70, 2, 9], [5, 300, 0, 64, 127]),
+    ([400], [0]), ([1] * 40, list(range(40, 80))), ([700, 1, 900], [0, 3, 130])])
+def test_attention_whole_and_in_units(ops, plain, heads, kv_heads, head_dim, page_size, portions,
+                                      histories):
+    """Against the plain function; then the same with the units of every token cut apart and with
+    none cut: the same bits. An infinite value that only later tokens see leaves earlier ones alone."""
+    ctx, table, pages = make_batch(portions, histories, page_size, DEVICE, seed=heads)
+    ctx.leading_single = next((i for i, n in enumerate(portions) if n > 1), len(portions))
+    generator = torch.Generator().manual_seed(head_dim)
+    kv = torch.randn(2, pages, kv_heads, page_size, head_dim, generator=generator)
+    q = torch.randn(ctx.tokens, heads, head_dim, generator=generator)
+    need = PagedKeyValues(kv_heads, head_dim, None)
+    view = PagedView(kv.to(DEVICE), table, page_size, need)
+    arguments = dict(heads=heads, kv_heads=kv_heads, head_dim=head_dim, scale=head_dim ** -0.5,
+                     window=None)
+    want = plain.paged_attention(q, ctx=on_cpu(ctx), view=PagedView(kv, table.cpu(), page_size, need),
+                                 **arguments)
+    got = ops.paged_attention(q.to(DEVICE), ctx=ctx, view=view, **arguments)
+    torch.testing.assert_close(got.cpu(), want, atol=2e-5, rtol=2e-5)
+    count, some = ops._sm_count, []
+    try:
+        for ops._sm_count in (0, 1 << 30):
+            some.append(ops.paged_attention(q.to(DEVICE), ctx=ctx, view=view, **arguments))
+    finally:
+        ops._sm_count = count
+    assert torch.equal(some[0], some[1]) and torch.equal(some[0], got)
+    ctx.leading_single = 0
+    assert torch.equal(ops.paged_attention(q.to(DEVICE), ctx=ctx, view=view, **arguments), got)
+    last = max(range(len(portions)), key=lambda r: portions[r])
+    if portions[last] > 1:
+        at = histories[last] + portions[last] - 1
+        view.kv[1, int(table[last, at // page_size]), :, at % page_size] = float("inf")
+        spoilt = ops.paged_attention(q.to(DEVICE), ctx=ctx, view=view, **arguments)
+        end = int(ctx.request_start[last + 1]) - 1
+        assert torch.isinf(spoilt[end]).all()
+        assert torch.equal(torch.cat((spoilt[:end], spoilt[end + 1:])), torch.cat((got[:end], got[end + 1:])))
+    ops.check_errors()
