@@ -32,6 +32,7 @@
 // its own channels are worked out in the block, the recurrence takes one pass, and the output's
 // norm and gate follow after a reduction over the block.
 #include "delta_common.cuh"
+#include "gated_delta_chunks.cuh"
 
 namespace {
 
@@ -501,6 +502,11 @@ delta_finish_kernel(const float* __restrict__ o, const T* __restrict__ projected
         mixed[item * V + e] = from_float<T>(row[e] * inv * weight[e] * silu(to_float<T>(gate[e])));
 }
 
+// (scratch and state are allocations of their own, so rows of q, k and v are aligned to 16 bytes)
+bool delta_in_chunks(int tokens, int requests, const DeltaSizes& sizes) {
+    return sizes.key_dim == DC_KEY && sizes.value_dim % DC_COLUMNS == 0 && tokens >= 8 * requests;
+}
+
 template <typename T>
 int launch_delta(const void* projected, const float* conv, const float* a_log, const float* dt_bias,
                  const float* norm_weight, float eps, float unit_eps, float* state,
@@ -544,6 +550,25 @@ int launch_delta(const void* projected, const float* conv, const float* a_log, c
                   (const T*)projected, conv, a_log, dt_bias, (const float*)state, slots,
                   token_request, request_start, history, q, k, v, coef, kq, sizes, unit_eps, ld);
     MLXONE_LAUNCH_CHECK("gated delta rule (prepare)");
+    // Keys of 128 values and portions of some length: 32 tokens at a time. A chunk takes the walk about
+    // as long as eight tokens take the scan below, so below eight tokens a request the scan is ahead.
+    float* chunks = kq + (size_t)tokens * G;
+    chunks += (4 - (chunks - scratch) % 4) % 4;
+    if (delta_in_chunks(tokens, requests, sizes)) {
+        cudaFuncSetAttribute(delta_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)DC_PREPARE_SHARED);
+        cudaFuncSetAttribute(delta_walk_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)DC_WALK_SHARED);
+        launch_kernel(delta_chunk_prepare_kernel, dim3(chunk_places(tokens, requests), G), dim3(DC_THREADS),
+                      DC_PREPARE_SHARED, stream, true, (const float*)q, (const float*)k, (const float*)coef,
+                      request_start, chunks, sizes, requests);
+        MLXONE_LAUNCH_CHECK("gated delta rule (chunks)");
+        launch_kernel(delta_walk_kernel<T>, dim3(V / DC_COLUMNS, H + 1, requests), dim3(DC_THREADS),
+                      DC_WALK_SHARED, stream, true, (const float*)q, (const float*)k, (const float*)v,
+                      (const float*)chunks, (const T*)projected, state, slots, request_start, history, o,
+                      sizes, write, ld);
+        MLXONE_LAUNCH_CHECK("gated delta rule (walk)");
+    } else {
     // A column's values are spread over 8 lanes (16 for keys longer than 128). Measured at 16 heads
     // of 128 x 128 and 2048 tokens: with 16 lanes every lane repeats the four tokens' solve for
     // half as many values of its own, 292 M warp instructions and 702 us.
@@ -568,6 +593,7 @@ int launch_delta(const void* projected, const float* conv, const float* a_log, c
     else SCAN(16, 16);
 #undef SCAN
     MLXONE_LAUNCH_CHECK("gated delta rule (scan)");
+    }
     const long long items = (long long)tokens * H;
     launch_kernel(delta_finish_kernel<T>, dim3(ceil_div_host(items, 8)), dim3(256), 0, stream, true,
                   (const float*)o, (const T*)projected, norm_weight, (T*)mixed, items, sizes, eps, ld);
@@ -577,11 +603,19 @@ int launch_delta(const void* projected, const float* conv, const float* a_log, c
 
 }  // namespace
 
+MLXONE_API int mlxone_gated_delta_in_chunks(int tokens, int requests, int heads, int kv_heads, int key_dim,
+                                            int value_dim) {
+    return delta_in_chunks(tokens, requests, {heads, kv_heads, key_dim, value_dim, 1});
+}
+
 // 32-bit values of scratch that a call with `tokens` tokens needs.
-MLXONE_API long long mlxone_gated_delta_scratch(int tokens, int heads, int kv_heads, int key_dim,
-                                                int value_dim) {
-    return (long long)tokens * (2LL * kv_heads * key_dim + 2LL * heads * value_dim + 2LL * heads +
-                                kv_heads);
+MLXONE_API long long mlxone_gated_delta_scratch(int tokens, int requests, int heads, int kv_heads,
+                                                int key_dim, int value_dim) {
+    const DeltaSizes sizes = {heads, kv_heads, key_dim, value_dim, 1};
+    const long long rows = (long long)tokens * (2LL * kv_heads * key_dim + 2LL * heads * value_dim +
+                                                2LL * heads + kv_heads);
+    if (!delta_in_chunks(tokens, requests, sizes)) return rows;
+    return rows + 4 + (long long)chunk_places(tokens, requests) * heads * DC_VALUES;
 }
 
 // 32-bit values of a request's slot.

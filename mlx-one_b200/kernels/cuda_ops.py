@@ -1275,8 +1275,8 @@ class CudaOps:
             raise KernelError(f"a state slot has {view.state[0].numel()} values, the mixer needs {size}")
         # a step of single tokens runs as one kernel, else preparation, scan and finish
         single = ctx.max_portion == 1 and tokens == ctx.requests
-        scratch = torch.empty(self.lib.mlxone_gated_delta_scratch(tokens, heads, kv_heads, key_dim,
-                                                                  value_dim),
+        scratch = torch.empty(self.lib.mlxone_gated_delta_scratch(tokens, ctx.requests, heads,
+                                                                  kv_heads, key_dim, value_dim),
                               dtype=torch.float32, device=self.device)
         out = torch.empty((tokens, inner), dtype=projected.dtype, device=self.device)
         self._call("mlxone_gated_delta", _c_void_p(_ptr(projected)), _c_void_p(_ptr(conv)),
@@ -1290,7 +1290,9 @@ class CudaOps:
                    _c_int(projected.stride(0)), _c_int(1 if single else 0),
                    _c_int(_dtype_code(projected.dtype)))
         if not (single and value_dim <= 128):
-            self.launches += 2
+            # preparation, scan and finish; chunks of long portions have a kernel more
+            self.launches += 2 + self.lib.mlxone_gated_delta_in_chunks(
+                tokens, ctx.requests, heads, kv_heads, key_dim, value_dim)
         return out
 
     def channel_delta_rule(self, projected, decay_up, gate_up, *, decay_columns, gate_columns, conv,

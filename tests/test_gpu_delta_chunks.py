@@ -1,0 +1,56 @@
+"""The gated delta rule over portions that are worked on 32 tokens at a time: portions at the edges of
+a chunk, several requests in a step, decays of zero, against the plain recurrence token by token."""
+
+import pytest
+import torch
+
+from test_gpu_galarax import DEVICE, DTYPES, bound, context, delta_pieces, ops  # noqa: F401  (fixture)
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads, kv_heads, value_dim", [(2, 1, 16), (3, 3, 48), (20, 2, 32)])
+@pytest.mark.parametrize("steps", [[(32, 40)], [(33, 31)], [(64, 1), (95, 65)], [(1, 70), (127, 3), (1, 30)]])
+@pytest.mark.parametrize("forget", [-5.0, 5.0])
+def test_portions_around_a_chunk(ops, dtype, heads, kv_heads, value_dim, steps, forget):
+    """``forget``: log of the decay's rate; at 5 most decays are zero in 32-bit."""
+    from mlx_one_b200.parts import FixedState, StateView
+    from mlx_one_b200.parts.mixers import GatedDeltaRule
+
+    H, G, D, V, taps = heads, kv_heads, 128, value_dim, 4
+    sizes = dict(heads=H, kv_heads=G, key_dim=D, value_dim=V, taps=taps)
+    channels, inner = 2 * G * D + H * V, H * V
+    width = channels + inner + 2 * H
+    generator = torch.Generator().manual_seed(V)
+    lengths = [sum(step[r] for step in steps) for r in (0, 1)]
+    projected = [(1.5 * torch.randn(n, width, generator=generator)).to(dtype) for n in lengths]
+    conv = 0.5 * torch.randn(channels, taps, generator=generator)
+    a_log = forget + torch.randn(H, generator=generator)
+    dt_bias, eps = torch.randn(H, generator=generator), 1e-5
+    norm_weight = 1 + 0.2 * torch.randn(V, generator=generator)
+    size = GatedDeltaRule.state_size(sizes)
+    state = torch.full((5, size), float("nan"), device=DEVICE)
+    state[[3, 1]] = 0
+    slots = torch.tensor([3, 1], dtype=torch.int32, device=DEVICE)
+    view = StateView(state, slots, FixedState((size,), "float32"))
+    constants = dict(conv=conv.to(DEVICE), a_log=a_log.to(DEVICE), dt_bias=dt_bias.to(DEVICE),
+                     norm_weight=norm_weight.to(DEVICE), eps=eps, unit_eps=1e-6, view=view, write=True,
+                     **sizes)
+    got, fed = [[], []], [0, 0]
+    for step in steps:
+        rows = torch.cat([projected[r][fed[r]:fed[r] + step[r]] for r in (0, 1)]).to(DEVICE)
+        before = ops.launches
+        out = ops.gated_delta_rule(rows, ctx=context(list(step), list(fed)), **constants)
+        assert ops.launches - before == 4          # preparation, chunks, walk, finish
+        got[0].append(out[:step[0]].cpu())
+        got[1].append(out[step[0]:].cpu())
+        fed = [fed[r] + step[r] for r in (0, 1)]
+    ops.check_errors()
+    for r in (0, 1):
+        want = delta_pieces(projected[r].double(), conv.double(), a_log.double(), dt_bias.double(),
+                            norm_weight.double(), eps, sizes)
+        difference = (torch.cat(got[r]).double() - want).abs().max()
+        # (the bounds of the recurrence's own test: 32-bit sums, 8 bits of mantissa at values of up to 8)
+        assert difference < bound(dtype, 5e-5, 0.1), f"request {r}: {difference}"
+    assert torch.isnan(state[[0, 2, 4]]).all() and torch.isfinite(state[[1, 3]]).all()
