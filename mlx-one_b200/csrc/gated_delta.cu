@@ -479,17 +479,24 @@ delta_scan_kernel(const float* __restrict__ q_in, const float* __restrict__ k_in
 
 // ------------------------------------------------------------------ a step of single tokens
 // One block per (value head, request); request r brings token r. Threads: STEP_LANES per column
-// of S. Dynamic shared memory: q and k [ROWS each], v and o [V each], four scalars.
+// of S. Dynamic shared memory: q and k [ROWS each], v and o [V each].
+//
+// Bound by latency (8 requests of 8 heads: 8 MB). So all that earlier steps left, the head's matrix, the
+// ring and the constants, is asked for before the wait for the kernel that writes this step's projection;
+// 64 registers a thread let the block lie beside that kernel's; what is read behind the wait is asked for
+// at once; and every warp works the few sums over a head out for itself, which leaves two barriers.
+// (Loads where their values were used, one warp's sums between four barriers and 128 registers: 9.7 us.)
 template <typename T, int PER>
-__global__ void __launch_bounds__(STEP_LANES * STEP_MAX_COLUMNS)
-delta_step_kernel(const T* __restrict__ projected, const float* __restrict__ conv,
+__global__ void __launch_bounds__(STEP_LANES * STEP_MAX_COLUMNS, PER <= 32 ? 2 : 1)
+delta_step_kernel(const T* projected, const float* __restrict__ conv,
                   const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                   const float* __restrict__ norm_weight, float eps, float unit_eps,
-                  float* __restrict__ state, const int* __restrict__ slots,
+                  float* state, const int* __restrict__ slots,
                   const int* __restrict__ history, T* __restrict__ mixed, DeltaSizes sizes,
                   int write, int ld) {
     constexpr int LANES = STEP_LANES;
     constexpr int ROWS = PER * LANES;
+    constexpr int HELD_TAPS = 4;
     extern __shared__ __align__(16) float staged[];
     const int H = sizes.heads, G = sizes.kv_heads, D = sizes.key_dim, V = sizes.value_dim;
     const int taps = sizes.taps, channels = sizes.channels();
@@ -497,38 +504,68 @@ delta_step_kernel(const T* __restrict__ projected, const float* __restrict__ con
     float* ks = qs + ROWS;
     float* vs = ks + ROWS;
     float* os = vs + V;
-    float* scalars = os + V;                 // k.q, decay, beta, 1 / rms(o)
     griddep_launch();
     const int h = blockIdx.x, r = blockIdx.y, g = h / (H / G);
     const int lane = threadIdx.x & (LANES - 1), column = threadIdx.x / LANES;
     const bool live = column < V;
-    // the head's matrix was written by an earlier step: its loads start before the wait for
-    // the kernel that writes this step's projection
     float* slot = state + (size_t)slots[r] * sizes.state();
     float* matrix = slot + (size_t)h * D * V;
     float S[PER];
+    {
+        const float* from = matrix + (size_t)(lane * 4) * V + column;
 #pragma unroll
-    for (int e = 0; e < PER; ++e) {
-        const int row = (e / 4) * (4 * LANES) + lane * 4 + e % 4;
-        S[e] = live && row < D ? matrix[(size_t)row * V + column] : 0.f;
+        for (int e = 0; e < PER; e += 4, from += (size_t)(4 * LANES) * V)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) S[e + i] = live && e * LANES + lane * 4 + i < D ? from[(size_t)i * V] : 0.f;
     }
+    const int t = r, position = history[r];
+    float* ring = slot + sizes.matrices();
+    // this block's channels: its key head's q and k, its own v
+    const int mine = 2 * D + V;
+    auto channel = [&](int i) {
+        return i < D ? g * D + i : i < 2 * D ? sizes.qk() + g * D + (i - D) : 2 * sizes.qk() + h * V + (i - 2 * D);
+    };
+    auto before_now = [&](int c, int j) {             // the input taps - 1 - j positions back
+        const int before = position - (taps - 1 - j);
+        return before >= 0 ? ring[(size_t)(before % taps) * channels + c] : 0.f;
+    };
+    // (the thread's first channel's weights and past, for kernels of up to four taps)
+    float weight[HELD_TAPS], past[HELD_TAPS - 1];
+    if ((int)threadIdx.x < mine && taps <= HELD_TAPS) {
+        const int c = channel(threadIdx.x);
+#pragma unroll
+        for (int j = 0; j < HELD_TAPS; ++j)
+            if (j < taps) weight[j] = conv[(size_t)c * taps + j];
+#pragma unroll
+        for (int j = 0; j < HELD_TAPS - 1; ++j)
+            if (j + 1 < taps) past[j] = before_now(c, j);
+    }
+    const float rate = a_log[h], bias = dt_bias[h];
+    const float norm = (int)threadIdx.x < V ? norm_weight[threadIdx.x] : 0.f;
     for (int i = threadIdx.x; i < 2 * ROWS; i += blockDim.x) qs[i] = 0.f;      // q and k, padded
     __syncthreads();
     griddep_wait();
-    const int t = r, position = history[r];
-    float* ring = slot + sizes.matrices();
     const T* row_in = projected + (size_t)t * ld;
-    // convolution + silu of this block's channels: its key head's q and k, its own v
+    const T* tail = row_in + channels + sizes.inner();
+    const float beta_in = to_float<T>(tail[h]), decay_in = to_float<T>(tail[H + h]);
+    const float gate = (int)threadIdx.x < V ? to_float<T>(row_in[channels + (size_t)h * V + threadIdx.x]) : 0.f;
+    // convolution + silu
     const bool owner = h % (H / G) == 0;         // writes the key head's inputs into the ring
-    for (int i = threadIdx.x; i < 2 * D + V; i += blockDim.x) {
-        const int c = i < D ? g * D + i : (i < 2 * D ? sizes.qk() + g * D + (i - D)
-                                                     : 2 * sizes.qk() + h * V + (i - 2 * D));
+    for (int i = threadIdx.x; i < mine; i += blockDim.x) {
+        const int c = channel(i);
         const float now = to_float<T>(row_in[c]);
-        float y = conv[(size_t)c * taps + taps - 1] * now;
-        for (int j = 0; j + 1 < taps; ++j) {
-            const int before = position - (taps - 1 - j);
-            if (before >= 0)
-                y = fmaf(conv[(size_t)c * taps + j], ring[(size_t)(before % taps) * channels + c], y);
+        float y;
+        if (i == (int)threadIdx.x && taps <= HELD_TAPS) {
+            y = 0.f;
+#pragma unroll
+            for (int j = 0; j < HELD_TAPS; ++j)
+                if (j + 1 == taps) y = weight[j] * now;
+#pragma unroll
+            for (int j = 0; j < HELD_TAPS - 1; ++j)
+                if (j + 1 < taps) y = fmaf(weight[j], past[j], y);
+        } else {
+            y = conv[(size_t)c * taps + taps - 1] * now;
+            for (int j = 0; j + 1 < taps; ++j) y = fmaf(conv[(size_t)c * taps + j], before_now(c, j), y);
         }
         if (write && (i >= 2 * D || owner)) ring[(size_t)(position % taps) * channels + c] = now;
         const float value = silu(y);
@@ -536,43 +573,27 @@ delta_step_kernel(const T* __restrict__ projected, const float* __restrict__ con
         else if (i < 2 * D) ks[i - D] = value;
         else vs[i - 2 * D] = value;
     }
+    const float decay = expf(-expf(rate) * softplus(decay_in + bias));
+    const float beta = 1.f / (1.f + expf(-beta_in));
     __syncthreads();
-    const int warp = threadIdx.x >> 5, in_warp = threadIdx.x & 31;
-    if (warp == 0) {
-        float qq = 0.f, kk = 0.f;
-        for (int e = in_warp; e < D; e += 32) {
-            qq = fmaf(qs[e], qs[e], qq);
-            kk = fmaf(ks[e], ks[e], kk);
-        }
-        qq = warp_sum(qq);
-        kk = warp_sum(kk);
-        const float q_scale = rsqrtf((float)D) / sqrtf(qq + unit_eps);
-        const float k_scale = 1.f / sqrtf(kk + unit_eps);
-        float dot = 0.f;
-        for (int e = in_warp; e < D; e += 32) {
-            const float qv = qs[e] * q_scale, kv = ks[e] * k_scale;
-            qs[e] = qv;
-            ks[e] = kv;
-            dot = fmaf(qv, kv, dot);
-        }
-        dot = warp_sum(dot);
-        if (in_warp == 0) {
-            scalars[0] = dot;
-            const T* tail = row_in + channels + sizes.inner();
-            scalars[1] = expf(-expf(a_log[h]) * softplus(to_float<T>(tail[H + h]) + dt_bias[h]));
-            scalars[2] = 1.f / (1.f + expf(-to_float<T>(tail[h])));
-        }
+    const int in_warp = threadIdx.x & 31;
+    // q and k to unit length (q also times D^-1/2): factors on what is summed with them
+    float qq = 0.f, kk = 0.f, qk = 0.f;
+    for (int e = in_warp; e < D; e += 32) {
+        qq = fmaf(qs[e], qs[e], qq);
+        kk = fmaf(ks[e], ks[e], kk);
+        qk = fmaf(qs[e], ks[e], qk);
     }
-    __syncthreads();
+    const float q_scale = rsqrtf((float)D) / sqrtf(warp_sum(qq) + unit_eps);
+    const float k_scale = 1.f / sqrtf(warp_sum(kk) + unit_eps);
+    qk = warp_sum(qk) * q_scale * k_scale;
     {
-        float k[PER];
         float wk[4] = {0.f, 0.f, 0.f, 0.f}, wq[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int e = 0; e < PER; e += 4) {
             const int at = (e / 4) * (4 * LANES) + lane * 4;
             const float4 k4 = *reinterpret_cast<const float4*>(ks + at);
             const float4 q4 = *reinterpret_cast<const float4*>(qs + at);
-            k[e] = k4.x; k[e + 1] = k4.y; k[e + 2] = k4.z; k[e + 3] = k4.w;
             wk[0] = fmaf(S[e], k4.x, wk[0]); wq[0] = fmaf(S[e], q4.x, wq[0]);
             wk[1] = fmaf(S[e + 1], k4.y, wk[1]); wq[1] = fmaf(S[e + 1], q4.y, wq[1]);
             wk[2] = fmaf(S[e + 2], k4.z, wk[2]); wq[2] = fmaf(S[e + 2], q4.z, wq[2]);
@@ -585,29 +606,31 @@ delta_step_kernel(const T* __restrict__ projected, const float* __restrict__ con
             with_k += __shfl_xor_sync(0xffffffffu, with_k, across);
             with_q += __shfl_xor_sync(0xffffffffu, with_q, across);
         }
-        const float decay = scalars[1];
-        const float u = scalars[2] * ((live ? vs[column] : 0.f) - decay * with_k);
+        const float u = beta * ((live ? vs[column] : 0.f) - decay * (k_scale * with_k));
+        if (live && lane == 0) os[column] = fmaf(u, qk, decay * (q_scale * with_q));
         if (write && live) {
+            const float moved = u * k_scale;
+            // (worked out anew: the addresses of the loads would not fit beside the column)
+            float* to = settled(matrix) + (size_t)(lane * 4) * V + column;
 #pragma unroll
-            for (int e = 0; e < PER; ++e) {
-                const int row = (e / 4) * (4 * LANES) + lane * 4 + e % 4;
-                if (row < D) matrix[(size_t)row * V + column] = fmaf(k[e], u, decay * S[e]);
+            for (int e = 0; e < PER; e += 4, to += (size_t)(4 * LANES) * V) {
+                const int at = e * LANES + lane * 4;
+                const float4 k4 = *reinterpret_cast<const float4*>(ks + at);
+                const float k[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (at + i < D) to[(size_t)i * V] = fmaf(k[i], moved, decay * S[e + i]);
             }
         }
-        if (live && lane == 0) os[column] = fmaf(u, scalars[0], decay * with_q);
     }
     __syncthreads();
-    if (warp == 0) {
-        float sum = 0.f;
-        for (int e = in_warp; e < V; e += 32) sum = fmaf(os[e], os[e], sum);
-        sum = warp_sum(sum);
-        if (in_warp == 0) scalars[3] = 1.f / sqrtf(sum / (float)V + eps);
-    }
-    __syncthreads();
-    const T* gate = row_in + channels + (size_t)h * V;
-    for (int e = threadIdx.x; e < V; e += blockDim.x)
-        mixed[(size_t)t * sizes.inner() + (size_t)h * V + e] =
-            from_float<T>(os[e] * scalars[3] * norm_weight[e] * silu(to_float<T>(gate[e])));
+    if ((int)(threadIdx.x & ~31u) >= V) return;
+    float sum = 0.f;
+    for (int e = in_warp; e < V; e += 32) sum = fmaf(os[e], os[e], sum);
+    const float inverse = 1.f / sqrtf(warp_sum(sum) / (float)V + eps);
+    if ((int)threadIdx.x < V)
+        mixed[(size_t)t * sizes.inner() + (size_t)h * V + threadIdx.x] =
+            from_float<T>(os[threadIdx.x] * inverse * norm * silu(gate));
 }
 
 // ------------------------------------------------------------------ finish
@@ -650,7 +673,7 @@ int launch_delta(const void* projected, const float* conv, const float* a_log, c
     if (single && tokens == requests && V <= STEP_MAX_COLUMNS) {
         // every request brings one token: one kernel
         const int per = D <= 16 ? 4 : D <= 32 ? 8 : D <= 64 ? 16 : D <= 128 ? 32 : 64;
-        const size_t shared = (size_t)(2 * per * STEP_LANES + 2 * V + 4) * sizeof(float);
+        const size_t shared = (size_t)(2 * per * STEP_LANES + 2 * V) * sizeof(float);
         const int threads = (STEP_LANES * V + 31) / 32 * 32;
 #define STEP(PER)                                                                              \
     launch_kernel(delta_step_kernel<T, PER>, dim3(H, requests), dim3(threads), shared, stream, \
