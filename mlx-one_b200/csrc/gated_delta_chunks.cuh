@@ -11,7 +11,6 @@
 // all chunks side by side; the walk over the chunks is then three products a chunk and five barriers
 // instead of a chain of sums and shuffles per four tokens. All in 32-bit; decays are multiplied up and
 // never divided, so a decay of zero is like any other.
-// (16 heads of 128 x 128, 2,048 tokens: see the walk below.)
 #pragma once
 
 #include "delta_common.cuh"
@@ -43,6 +42,16 @@ __device__ __forceinline__ FloatPair pair_of(float x) {
     asm("mov.b64 %0, {%1, %1};" : "=l"(p) : "f"(x));
     return p;
 }
+__device__ __forceinline__ FloatPair pair_of(float x, float y) {
+    FloatPair p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(x), "f"(y));
+    return p;
+}
+__device__ __forceinline__ FloatPair mul_pair(FloatPair x, FloatPair y) {
+    FloatPair p;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(x), "l"(y));
+    return p;
+}
 __device__ __forceinline__ void fma_pair(FloatPair& acc, FloatPair x, FloatPair y) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y));
 }
@@ -57,18 +66,20 @@ __device__ __forceinline__ float4 quad_of(FloatPair a, FloatPair b) {
 // Grid (chunk places, query/key heads). The products of the chunk's k and q with its k: a warp takes 16
 // of the 128 values of a key, a lane 8 x 8 products (16 values read from shared memory for 64 FMAs:
 // shared memory gives a thread's value for every four FMAs that an SM can do); then a warp per value
-// head, lane = column: T by forward substitution in registers, P T behind it.
-constexpr size_t DC_PREPARE_SHARED =
-    sizeof(float) * ((size_t)2 * DC * DC_PITCH + 8 * 2 * DC * DC + 8 * 2 * DC * DC_SMALL);
+// head, lane = column: T by forward substitution in registers, P T behind it. (A and P of up to three
+// heads lie where k and q lay, so that two blocks share an SM: room for eight of them beside k and q left
+// one: 31 us for 2,048 tokens of 16 heads, 24 now.)
+constexpr int DC_SOLVERS = 3;
+constexpr size_t DC_PREPARE_SHARED = sizeof(float) * ((size_t)2 * DC * DC_PITCH + 8 * 2 * DC * DC);
+static_assert(DC_SOLVERS * 2 * DC * DC_SMALL <= 2 * DC * DC_PITCH, "A and P fit where k and q were");
 
-__global__ void __launch_bounds__(DC_THREADS)
+__global__ void __launch_bounds__(DC_THREADS, 2)
 delta_chunk_prepare_kernel(const float* q_in, const float* k_in, const float* coef,
                            const int* __restrict__ request_start, float* chunks, DeltaSizes sizes,
                            int requests) {
     extern __shared__ __align__(16) float shared[];
     float* kq = shared;                                      // [k of 32 tokens, q of 32][DC_PITCH]
     float* part = kq + 2 * DC * DC_PITCH;                    // [8][64][32]
-    float* small = part + 8 * 2 * DC * DC;                   // per warp: A, P [32][DC_SMALL] each
     __shared__ int place[2];                                 // first token, tokens
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = blockIdx.y;
     const int H = sizes.heads, G = sizes.kv_heads, per_group = H / G;
@@ -135,9 +146,10 @@ delta_chunk_prepare_kernel(const float* q_in, const float* k_in, const float* co
         part[i] = sum;
     }
     __syncthreads();
-    float* a = small + warp * 2 * DC * DC_SMALL;
+    if (warp >= DC_SOLVERS) return;
+    float* a = kq + warp * 2 * DC * DC_SMALL;
     float* p = a + DC * DC_SMALL;
-    for (int hh = warp; hh < per_group; hh += 8) {
+    for (int hh = warp; hh < per_group; hh += DC_SOLVERS) {
         const int h = g * per_group + hh;
         float gate = 1.f, beta = 0.f;                        // (behind the portion's end: changes nothing)
         if (lane < count) {
@@ -200,11 +212,14 @@ delta_chunk_prepare_kernel(const float* q_in, const float* k_in, const float* co
 // convolution's inputs into the ring. S lies in shared memory (and in the registers of the 128 threads
 // that update it). [k; q] S and [T diag(beta); P T diag(beta)] r are products of 64 rows by 16 columns: a
 // lane takes 8 x 4 outputs, a warp an eighth of the sum (16 values of a key, 4 tokens), and the eighths
-// are added up in order. Bound by shared memory's 32 values a cycle: a chunk reads about 110,000
-// values. The next chunk's operands travel while this one is worked on.
+// are added up in order. Bound by the chain of products, barriers and reads of shared memory of a chunk
+// (2.6 us; 56 % of the SMs' shared memory reads, 40 % of their FMAs): tiles of 8 columns and twice the
+// blocks were 5 to 10 % slower, for 4 heads too. While half the warps update S the other half asks for the
+// chunk after next. 2,048 tokens of 16 heads: 170 us (530 by the scan of four tokens at a time).
+constexpr int DC_BUFFERS = 3;
 constexpr int DC_BUFFER = 2 * DC * DC_PITCH + DC * DC_COLUMNS + 2 * DC * DC_SMALL + 2 * DC;
 constexpr size_t DC_WALK_SHARED =
-    sizeof(float) * ((size_t)2 * DC_BUFFER + DC_KEY * DC_COLUMNS + 8 * 2 * DC * DC_COLUMNS + 2 * DC * DC_COLUMNS);
+    sizeof(float) * ((size_t)DC_BUFFERS * DC_BUFFER + DC_KEY * DC_COLUMNS + 8 * 2 * DC * DC_COLUMNS + 2 * DC * DC_COLUMNS);
 
 // part[warp][64][16] = x[64 rows, 4 STEPS columns from e0] * y[4 STEPS rows, 16 columns]
 template <int STEPS>
@@ -244,7 +259,7 @@ delta_walk_kernel(const float* q_in, const float* k_in, const float* v_in, const
                   const int* __restrict__ request_start, const int* __restrict__ history, float* out,
                   DeltaSizes sizes, int write, int ld) {
     extern __shared__ __align__(16) float shared[];
-    float* matrix_s = shared + 2 * DC_BUFFER;                // S [128][16]
+    float* matrix_s = shared + DC_BUFFERS * DC_BUFFER;       // S [128][16]
     float* part = matrix_s + DC_KEY * DC_COLUMNS;            // [8][64][16]
     float* rest = part + 8 * 2 * DC * DC_COLUMNS;            // r [32][16]
     float* moved = rest + DC * DC_COLUMNS;                   // D(32, t) u_t [32][16]
@@ -266,43 +281,49 @@ delta_walk_kernel(const float* q_in, const float* k_in, const float* v_in, const
         return;
     }
     const int h = blockIdx.y, g = h / (H / G), column0 = blockIdx.x * DC_COLUMNS;
-    auto fetch = [&](int chunk, float* to) {
+    // the chunk's operands into its buffer, by `count_of` threads of which this is number `me`; a group of
+    // copies even where there is no such chunk
+    auto fetch = [&](int chunk, int me, int count_of) {
+        if (first + chunk * DC >= last) { copy_commit(); return; }
+        float* to = shared + chunk % DC_BUFFERS * DC_BUFFER;
         const int base = first + chunk * DC, count = min(DC, last - base);
-        for (int i = tid; i < 2 * DC * (DC_KEY / 4); i += DC_THREADS) {
+        for (int i = me; i < 2 * DC * (DC_KEY / 4); i += count_of) {
             const int row = i / (DC_KEY / 4), e = i % (DC_KEY / 4) * 4, t = row % DC;
             copy_or_zero_16(to + row * DC_PITCH + e,
                             (row < DC ? k_in : q_in) + ((size_t)(base + min(t, count - 1)) * G + g) * DC_KEY + e,
                             t < count);
         }
         to += 2 * DC * DC_PITCH;
-        if (tid < DC * (DC_COLUMNS / 4)) {
-            const int t = tid / (DC_COLUMNS / 4), c = tid % (DC_COLUMNS / 4) * 4;
+        if (me < DC * (DC_COLUMNS / 4)) {
+            const int t = me / (DC_COLUMNS / 4), c = me % (DC_COLUMNS / 4) * 4;
             copy_or_zero_16(to + t * DC_COLUMNS + c,
                             v_in + ((size_t)(base + min(t, count - 1)) * H + h) * V + column0 + c, t < count);
         }
         to += DC * DC_COLUMNS;
         const float* from = chunks + ((size_t)(first_chunk(first, r) + chunk) * H + h) * DC_VALUES;
-        for (int i = tid; i < 2 * DC * (DC / 4); i += DC_THREADS) {
+        for (int i = me; i < 2 * DC * (DC / 4); i += count_of) {
             const int row = i / (DC / 4), e = i % (DC / 4) * 4;
             copy_or_zero_16(to + row * DC_SMALL + e, from + row * DC + e, true);
         }
         to += 2 * DC * DC_SMALL;
-        if (tid < 2 * DC / 4) copy_or_zero_16(to + tid * 4, from + 2 * DC * DC + tid * 4, true);
+        if (me < 2 * DC / 4) copy_or_zero_16(to + me * 4, from + 2 * DC * DC + me * 4, true);
         copy_commit();
     };
     const int total = (last - first + DC - 1) / DC;
-    if (total > 0) fetch(0, shared);
+    fetch(0, tid, DC_THREADS);
+    fetch(1, tid, DC_THREADS);
     // S: thread t < 128 keeps rows 4 (t / 4) .. + 3 of columns 4 (t % 4) .. + 3
     const int own_row = tid / 4 * 4, own_column = tid % 4 * 4;
     float* matrix = slot + (size_t)h * DC_KEY * V + column0;
-    float S[4][4];
+    FloatPair S[4][2];
     if (tid < 128) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) S[i][j] = matrix[(size_t)(own_row + i) * V + own_column + j];
+            const float* from = matrix + (size_t)(own_row + i) * V + own_column;
+            S[i][0] = pair_of(from[0], from[1]);
+            S[i][1] = pair_of(from[2], from[3]);
             *reinterpret_cast<float4*>(matrix_s + (own_row + i) * DC_COLUMNS + own_column) =
-                make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+                quad_of(S[i][0], S[i][1]);
         }
     }
     // sums of the eighths: thread t adds up four columns of row t / 4
@@ -318,13 +339,12 @@ delta_walk_kernel(const float* q_in, const float* k_in, const float* v_in, const
         return sum;
     };
     for (int chunk = 0; chunk < total; ++chunk) {
-        const float* kq = shared + (chunk & 1) * DC_BUFFER;
+        const float* kq = shared + chunk % DC_BUFFERS * DC_BUFFER;
         const float* vs = kq + 2 * DC * DC_PITCH;
         const float* small = vs + DC * DC_COLUMNS;
         const float* decays = small + 2 * DC * DC_SMALL;     // G_t, D(32, t)
-        copy_wait_for<0>();
+        copy_wait_for<1>();                                  // (the chunk behind this one may be under way)
         __syncthreads();
-        if (chunk + 1 < total) fetch(chunk + 1, shared + ((chunk + 1) & 1) * DC_BUFFER);
         chunk_product<4>(kq + warp * 16, DC_PITCH, matrix_s + warp * 16 * DC_COLUMNS,
                          part + warp * 2 * DC * DC_COLUMNS);
         __syncthreads();
@@ -353,33 +373,40 @@ delta_walk_kernel(const float* q_in, const float* k_in, const float* v_in, const
         }
         __syncthreads();
         if (tid < 128) {
-            const float whole = decays[DC - 1];
+            // (half the warps, the other half asks for the chunk after next meanwhile)
+            const FloatPair whole = pair_of(decays[DC - 1]);
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) S[i][j] *= whole;
+                for (int j = 0; j < 2; ++j) S[i][j] = mul_pair(S[i][j], whole);
 #pragma unroll 8
             for (int t = 0; t < DC; ++t) {
                 const float4 k = *reinterpret_cast<const float4*>(kq + t * DC_PITCH + own_row);
-                const float4 u = *reinterpret_cast<const float4*>(moved + t * DC_COLUMNS + own_column);
-                const float ks[4] = {k.x, k.y, k.z, k.w}, us[4] = {u.x, u.y, u.z, u.w};
+                const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(moved + t * DC_COLUMNS + own_column);
+                const FloatPair ks[4] = {pair_of(k.x), pair_of(k.y), pair_of(k.z), pair_of(k.w)};
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) S[i][j] = fmaf(ks[i], us[j], S[i][j]);
+                for (int i = 0; i < 4; ++i) {
+                    fma_pair(S[i][0], ks[i], u.x);
+                    fma_pair(S[i][1], ks[i], u.y);
+                }
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
                 *reinterpret_cast<float4*>(matrix_s + (own_row + i) * DC_COLUMNS + own_column) =
-                    make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+                    quad_of(S[i][0], S[i][1]);
+            copy_commit();                                   // (groups are counted thread by thread)
+        } else {
+            fetch(chunk + 2, tid - 128, 128);
         }
     }
     griddep_launch();
     if (write && tid < 128) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) matrix[(size_t)(own_row + i) * V + own_column + j] = S[i][j];
+        for (int i = 0; i < 4; ++i) {
+            const float4 v = quad_of(S[i][0], S[i][1]);
+            float* to = matrix + (size_t)(own_row + i) * V + own_column;
+            to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w;
+        }
     }
 }
 
