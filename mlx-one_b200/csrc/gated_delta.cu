@@ -125,6 +125,7 @@ template <typename T> struct FourOf;
 template <> struct FourOf<float> {
     using Raw = float4;
     static __device__ __forceinline__ float4 wide(const Raw& v) { return v; }
+    static __device__ __forceinline__ Raw narrow(const float4& v) { return v; }
 };
 template <> struct FourOf<__nv_bfloat16> {
     using Raw = uint2;
@@ -132,6 +133,13 @@ template <> struct FourOf<__nv_bfloat16> {
         const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&v.x);
         const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&v.y);
         return make_float4(__low2float(lo), __high2float(lo), __low2float(hi), __high2float(hi));
+    }
+    static __device__ __forceinline__ Raw narrow(const float4& v) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+        Raw raw;
+        raw.x = *reinterpret_cast<const uint32_t*>(&lo);
+        raw.y = *reinterpret_cast<const uint32_t*>(&hi);
+        return raw;
     }
 };
 
@@ -639,7 +647,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 delta_finish_kernel(const float* __restrict__ o, const T* __restrict__ projected,
                     const float* __restrict__ weight, T* __restrict__ mixed, long long items,
-                    DeltaSizes sizes, float eps, int ld) {
+                    DeltaSizes sizes, float eps, int ld, bool fours) {
     griddep_launch();
     griddep_wait();
     const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -651,6 +659,19 @@ delta_finish_kernel(const float* __restrict__ o, const T* __restrict__ projected
     const float* row = o + item * V;
     const T* gate = projected + (size_t)t * ld + sizes.channels() + (size_t)h * V;
     float sum = 0.f;
+    if (fours) {
+        // (128 values, all aligned: four neighbouring ones a lane, asked for at once)
+        const float4 y = reinterpret_cast<const float4*>(row)[lane];
+        const auto raw = reinterpret_cast<const typename FourOf<T>::Raw*>(gate)[lane];
+        const float4 w = reinterpret_cast<const float4*>(weight)[lane];
+        const float4 z = FourOf<T>::wide(raw);
+        sum = warp_sum(fmaf(y.w, y.w, fmaf(y.z, y.z, fmaf(y.y, y.y, y.x * y.x))));
+        const float inv = 1.f / sqrtf(sum / 128.f + eps);
+        reinterpret_cast<typename FourOf<T>::Raw*>(mixed + item * 128)[lane] =
+            FourOf<T>::narrow(make_float4(y.x * inv * w.x * silu(z.x), y.y * inv * w.y * silu(z.y),
+                                          y.z * inv * w.z * silu(z.z), y.w * inv * w.w * silu(z.w)));
+        return;
+    }
     for (int e = lane; e < V; e += 32) sum = fmaf(row[e], row[e], sum);
     sum = warp_sum(sum);
     const float inv = 1.f / sqrtf(sum / (float)V + eps);
@@ -763,7 +784,9 @@ int launch_delta(const void* projected, const float* conv, const float* a_log, c
     }
     const long long items = (long long)tokens * H;
     launch_kernel(delta_finish_kernel<T>, dim3(ceil_div_host(items, 8)), dim3(256), 0, stream, true,
-                  (const float*)o, (const T*)projected, norm_weight, (T*)mixed, items, sizes, eps, ld);
+                  (const float*)o, (const T*)projected, norm_weight, (T*)mixed, items, sizes, eps, ld,
+                  V == 128 && ld % 4 == 0 && sizes.channels() % 4 == 0 &&
+                      aligned(projected) && aligned(norm_weight) && aligned(mixed) && aligned(o));
     MLXONE_LAUNCH_CHECK("gated delta rule (finish)");
     return 0;
 }
