@@ -29,6 +29,7 @@ using bf16 = __nv_bfloat16;
 constexpr int BM = 128;
 constexpr int BK = 64;                 // 64 bf16 = 128 bytes: one swizzle row
 constexpr int WIDE_STAGES = 4;         // 128 x 256 tiles: 4 x 48 KB
+constexpr int MIDDLE_STAGES = 5;       // 128 x 192 tiles: 5 x 40 KB
 constexpr int NARROW_STAGES = 6;       // 128 x 128 tiles: 6 x 32 KB
 constexpr int THREADS = 192;           // producer warp, mma warp, four epilogue warps
 constexpr int WAIT_LIMIT = 1 << 24;    // polls before a wait gives up
@@ -145,6 +146,9 @@ __host__ __device__ constexpr uint32_t instruction_descriptor(int m, int n) {
            ((uint32_t)(m >> 4) << 24);
 }
 
+// Two accumulators of BN columns; tensor memory is given out in powers of two.
+__host__ __device__ constexpr int tmem_columns(int bn) { return bn <= 128 ? 256 : 512; }
+
 template <int BN, int EPILOGUE, int STAGES>
 __global__ void __launch_bounds__(THREADS)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
@@ -185,7 +189,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(shared_address(&tmem_base_slot), 2 * BN);
+    if (warp == 1) tmem_alloc(shared_address(&tmem_base_slot), tmem_columns(BN));
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
@@ -400,7 +404,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
             // shared memory before the block ends
             for (int i = 0; i < 1000; ++i) __nanosleep(1000);
         }
-        tmem_free(tmem_base, 2 * BN);
+        tmem_free(tmem_base, tmem_columns(BN));
     }
 }
 
@@ -446,6 +450,22 @@ struct Grouping {
     int out_limit = 0;
 };
 
+int sm_count() {
+    if (g_sm_count == 0) {
+        int device = 0;
+        cudaGetDevice(&device);
+        cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, device);
+        if (g_sm_count <= 0) g_sm_count = 148;
+    }
+    return g_sm_count;
+}
+
+// How many tiles of 128 rows by `columns` an SM works through for a gated product.
+int gated_rounds(int m, int width, int columns) {
+    const long long tiles = (long long)((m + BM - 1) / BM) * ((width + columns - 1) / columns);
+    return (int)((tiles + sm_count() - 1) / sm_count());
+}
+
 template <int BN, int EPILOGUE, int STAGES>
 int launch(const void* a, int lda, const void* w, const float* bias, void* out, int ldo, int m,
            int n, int k, int up_offset, int* error_flag, cudaStream_t stream,
@@ -464,13 +484,7 @@ int launch(const void* a, int lda, const void* w, const float* bias, void* out, 
     const int columns = grouped ? grouping.out_limit : EPILOGUE == SWIGLU ? up_offset : n;
     const int tiles_m = (m + BM - 1) / BM;
     const int total_tiles = tiles_m * ((columns + out_columns - 1) / out_columns);
-    if (g_sm_count == 0) {
-        int device = 0;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, device);
-        if (g_sm_count <= 0) g_sm_count = 148;
-    }
-    const dim3 grid(total_tiles < g_sm_count ? total_tiles : g_sm_count);
+    const dim3 grid(total_tiles < sm_count() ? total_tiles : sm_count());
     const size_t shared = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 1024 + 4 * 32 * 33 * 4;
     auto kernel = gemm_tcgen05_kernel<BN, EPILOGUE, STAGES>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -516,7 +530,14 @@ MLXONE_API int mlxone_gemm_tcgen05(const void* a, int lda, const void* w, const 
                         : launch<128, STORE_BF16, NARROW_STAGES>(a, lda, w, bias, out, ldo, m, n, k, 0, error_flag, stream);
             break;
         case SWIGLU:
-            code = launch<256, SWIGLU, WIDE_STAGES>(a, lda, w, bias, out, ldo, m, n, k, n / 2, error_flag, stream);
+            // Tiles of 96 + 96 instead of 128 + 128 rows of w where they take no more rounds over the
+            // SMs: 424 rows of 2 x 6,912 columns of 1,536 are two rounds of either, 24.6 against 28.2
+            // us; 528 rows of 2 x 8,192 columns of 2,048 three, 39.4 against 44.5 us. With a round more the
+            // operands' additional reads outweigh the smaller tiles (900 rows of the latter, five rounds
+            // against four: 58.6 against 56.5 us).
+            code = gated_rounds(m, n / 2, 96) <= gated_rounds(m, n / 2, 128)
+                       ? launch<192, SWIGLU, MIDDLE_STAGES>(a, lda, w, bias, out, ldo, m, n, k, n / 2, error_flag, stream)
+                       : launch<256, SWIGLU, WIDE_STAGES>(a, lda, w, bias, out, ldo, m, n, k, n / 2, error_flag, stream);
             break;
         case ADD_RESIDUAL:
             code = wide ? launch<256, ADD_RESIDUAL, WIDE_STAGES>(a, lda, w, bias, out, ldo, m, n, k, 0, error_flag, stream)
