@@ -25,7 +25,8 @@
 //            once per block) the four u and o follow from numbers alone; a second pass updates
 //            the column for all four. The operands of the next 16 tokens travel to shared
 //            memory (cp.async) while the current 16 are worked on. Extra blocks write the
-//            convolution's inputs into the ring.
+//            convolution's inputs into the ring. (Keys of 128 values and longer portions: 32 tokens at a
+//            time by two kernels, gated_delta_chunks.cuh.)
 //   finish   per (token, head): o / rms(o) * weight * silu(gate), in the compute type.
 // A step of single tokens runs one kernel, a block per (request, value head): the head's
 // matrix is asked for before the wait for the projection, the convolutions, norms and gates of
