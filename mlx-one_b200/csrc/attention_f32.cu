@@ -13,7 +13,8 @@
 // of 4 heads) for portions, RPT = 1 for single tokens. SPLIT: a block computes one unit, and a merge
 // kernel joins them: taken where there would be too few blocks to keep the chip busy. (One warp per
 // query and head, which reads every key for itself by a lane per key, 4-byte loads a head apart: 188
-// us a launch for one token behind 140 keys, 760 us for four prompts of 300.)
+// us a launch for one token behind 140 keys, 760 us for four prompts of 300; now 8 and 110. With the
+// rows looked up by every thread for itself and all loads behind the wait 12.5 and 130.)
 #include "common.cuh"
 
 namespace {
@@ -63,12 +64,51 @@ attention_f32_kernel(const float* q, const float* kv, const int* block_table, in
     float* values = keys + UNIT * PAD;                // [UNIT][D]
     float* queries = values + UNIT * D;               // [ROWS][PAD]
     float* weights = queries + ROWS * PAD;            // [ROWS][UNIT + 1]
-    __shared__ int dead[UNIT];                        // keys whose position has no page
+    __shared__ long long row_of[UNIT];                // where a key's row lies, -1: its position has no page
     const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
     const int group = heads / kv_heads, kv_head = blockIdx.y;
     const int token0 = first_token + blockIdx.x * tile_tokens;
     const int tokens_here = min(tile_tokens, end_token - token0);
-    griddep_wait();
+
+    // the rows of a unit's keys, looked up once; then keys low .. high - 1 of it, 16 bytes a thread
+    auto look_up = [&](const int* table, int base, int last) {
+        if (tid < UNIT) {
+            const int key = base + tid;
+            long long at = -1;
+            if (key <= last) {
+                const int block = key / page_size;
+                const int page = block < table_width ? __ldcg(table + block) : -1;
+                if (page < 0) atomicExch(error_flag, 3);
+                else at = (((long long)page * kv_heads + kv_head) * page_size + key % page_size) * D;
+            }
+            row_of[tid] = at;
+        }
+        __syncthreads();
+    };
+    auto bring = [&](int low, int high) {
+        for (int i = low * (D / 4) + tid; i < high * (D / 4); i += THREADS) {
+            const int j = i / (D / 4), e = i % (D / 4) * 4;
+            const long long at = row_of[j];
+            const float* from = at >= 0 ? kv + at + e : kv;
+            copy16(keys + j * PAD + e, from, at >= 0);
+            copy16(values + j * D + e, at >= 0 ? from + kv_half : kv, at >= 0);
+        }
+    };
+    // A single token's first unit: all keys but its own lie in the pages since earlier steps, so they are
+    // asked for ahead of the wait for the kernel that writes that one (positions and tables are older still).
+    bool ahead = false;
+    if (RPT == 1) {
+        const int last = __ldcg(positions + token0), base = SPLIT ? (int)blockIdx.z * UNIT : 0;
+        ahead = base <= last;
+        if (ahead) {
+            look_up(block_table + (size_t)__ldcg(token_request + token0) * table_width, base, last);
+            bring(0, min(last - base, UNIT));
+        }
+        griddep_wait();
+        if (ahead) bring(min(last - base, UNIT), UNIT);
+    } else {
+        griddep_wait();
+    }
     griddep_launch();
 
     // rows: row = (token of the tile) * group + head of the group
@@ -110,21 +150,10 @@ attention_f32_kernel(const float* q, const float* kv, const int* block_table, in
         const int end_unit = SPLIT ? min(first_unit + 1, last / UNIT + 1) : last / UNIT + 1;
         for (int unit = first_unit; unit < end_unit; ++unit) {
             const int base = unit * UNIT;
-            __syncthreads();                          // the unit before has been read
-            for (int i = tid; i < UNIT * (D / 4); i += THREADS) {
-                const int j = i / (D / 4), e = i % (D / 4) * 4, key = base + j;
-                int page = -1;
-                if (key <= last) {
-                    const int block = key / page_size;
-                    page = block < table_width ? __ldcg(table + block) : -1;
-                    if (page < 0) atomicExch(error_flag, 3);
-                }
-                const float* from = kv;
-                if (page >= 0)
-                    from = kv + (((size_t)page * kv_heads + kv_head) * page_size + key % page_size) * D + e;
-                copy16(keys + j * PAD + e, from, page >= 0);
-                copy16(values + j * D + e, page >= 0 ? from + kv_half : kv, page >= 0);
-                if (e == 0) dead[j] = page < 0;
+            if (!ahead || unit != first_unit) {
+                __syncthreads();                      // the unit before has been read
+                look_up(table, base, last);
+                bring(0, UNIT);
             }
             asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
             __syncthreads();
@@ -165,7 +194,7 @@ attention_f32_kernel(const float* q, const float* kv, const int* block_table, in
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const int j = tx + 16 * c;
-                    if (j >= seen[i] || dead[j]) score[i][c] = -INFINITY;
+                    if (j >= seen[i] || row_of[j] < 0) score[i][c] = -INFINITY;
                     most = fmaxf(most, score[i][c]);
                 }
                 unit_max[i] = half_max(most);
@@ -173,7 +202,7 @@ attention_f32_kernel(const float* q, const float* kv, const int* block_table, in
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const int j = tx + 16 * c;
-                    const bool live = j < seen[i] && !dead[j] && unit_max[i] != -INFINITY;
+                    const bool live = j < seen[i] && row_of[j] >= 0 && unit_max[i] != -INFINITY;
                     const float weight = live ? expf(score[i][c] - unit_max[i]) : 0.f;
                     weights[(ty * RPT + i) * (UNIT + 1) + j] = weight;
                     total += weight;
