@@ -280,15 +280,17 @@ attention_f32_kernel(const float* q, const float* kv, const int* block_table, in
     }
 }
 
-// One block of D threads per (token, head).
+// One block of D threads per (token, head). A position behind the units that were launched raises the
+// error flag, as a key without a page does.
 template <int D>
 __global__ void __launch_bounds__(D) attention_f32_merge_kernel(const float* partial, const int* positions,
                                                                 float* out, int units, int first_token,
-                                                                int heads) {
+                                                                int heads, int* error_flag) {
     griddep_wait();
     griddep_launch();
     const int item = blockIdx.x, d = threadIdx.x;
-    const int count = __ldcg(positions + first_token + item / heads) / UNIT + 1;
+    const int seen = __ldcg(positions + first_token + item / heads) / UNIT + 1, count = min(seen, units);
+    if (seen > units && d == 0) atomicExch(error_flag, 3);
     const float* from = partial + (size_t)item * units * (D + 4);
     float max_so_far = -INFINITY, sum = 0.f, acc = 0.f;
 #pragma unroll 4
@@ -328,7 +330,7 @@ void launch(const Arguments& x, int first, int end, int tile_tokens) {
                   tile_tokens, x.heads, x.kv_heads, x.scale, x.error_flag);
     if (SPLIT)
         launch_kernel(attention_f32_merge_kernel<D>, dim3((end - first) * x.heads), dim3(D), 0, x.stream, true,
-                      x.partial, x.positions, x.out, x.units, first, x.heads);
+                      x.partial, x.positions, x.out, x.units, first, x.heads, x.error_flag);
 }
 
 template <int D>
@@ -352,8 +354,8 @@ MLXONE_API int mlxone_attention_f32_supports(int head_dim, int heads, int kv_hea
 }
 
 // The tokens first .. end - 1 of a step. `single`: each of them is its request's only one. `units`: 0,
-// or an upper bound of the units of 64 keys that a token reads; then a block computes one unit and
-// `partial` holds (end - first) * heads * units * (head_dim + 4) values.
+// or an upper bound of the units of 64 keys that a token reads (one that reads more raises the error flag);
+// then a block computes one unit and `partial` holds (end - first) * heads * units * (head_dim + 4) values.
 MLXONE_API int mlxone_attention_f32(const float* q, const float* kv, const int* block_table, int table_width,
                                     int page_size, int pages, const int* positions, const int* token_request,
                                     float* out, float* partial, int first, int end, int single, int units,

@@ -369,7 +369,9 @@ class Runner:
         views = {entry: self.cache.view(entry, tables, slots) for entry in self.model.cache_needs}
         if captured is None or not self.use_graphs:
             max_portion = max(len(e.tokens) for e in entries)
-            max_context = max(c.length + len(e.tokens) for c, e in zip(caches, entries))
+            # (a loop's later steps run with this context too, their positions further on)
+            later = loop[0] - 1 if loop is not None else 0
+            max_context = max(c.length + len(e.tokens) for c, e in zip(caches, entries)) + later
             host = {"history": history, "request_start": starts}
         else:
             # bounds that hold for every step of this shape, however its tokens are split

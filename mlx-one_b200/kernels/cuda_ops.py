@@ -1729,7 +1729,9 @@ class CudaOps:
             singles = tokens
         else:
             singles = min(getattr(ctx, "leading_single", 0), ctx.requests)
-        units = -(-min(ctx.max_context, width * view.page_size) // 64)
+        # (all that a table can hold: whatever the device's positions are by the time this runs, one
+        # behind that has no page and raises the error flag)
+        units = -(-width * view.page_size // 64)
         group = heads // kv_heads
         for first, end, single in ((0, singles, 1), (singles, tokens, 0)):
             if first == end:

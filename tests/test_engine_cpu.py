@@ -89,6 +89,31 @@ def test_mixed_batches_reuse_pages(models, name):
     assert not cache.requests()
 
 
+def test_decode_loop_bounds_hold_for_every_step(models, monkeypatch):
+    """A loop of decode steps keeps one context while the positions move on the device: its
+    ``max_context`` covers the last step's, and the tokens are those of steps one by one."""
+    folder, loaded, plain = models["A"]
+    config, _, page = CONFIGS["A"]
+    runner, cache = runner_for(loaded, page, 256)
+    requests = prompts(config["vocab_size"], (30, 5), seed=14)
+    want = [plain.greedy(tokens, 13) for tokens in requests]
+    attention, seen = loaded.model.ops.paged_attention, []
+
+    def attend(q, *, ctx, view, **rest):
+        seen.append(int(ctx.positions.max()))
+        assert seen[-1] < ctx.max_context <= view.block_table.shape[1] * view.page_size
+        return attention(q, ctx=ctx, view=view, **rest)
+
+    for i, tokens in enumerate(requests):
+        cache.open(i)
+        runner.step([StepEntry(i, tokens)])
+    monkeypatch.setattr(loaded.model.ops, "paged_attention", attend)
+    got = runner.decode_steps([StepEntry(i, [w[0]]) for i, w in enumerate(want)], 12)
+    assert got.T.tolist() == [w[1:] for w in want] and max(seen) == 41
+    for i in range(len(requests)):
+        cache.close(i)
+
+
 def test_step_refuses_bad_batches_before_touching_state(models):
     folder, loaded, plain = models["A"]
     runner, cache = runner_for(loaded, 4, 32)

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from test_gpu_kernels import make_batch, on_cpu, ops, plain  # noqa: F401  (fixtures)
+from tiny_models import CONFIGS, make_model_dir, prompts
 from mlx_one_b200.parts.base import PagedKeyValues, PagedView
 
 pytestmark = pytest.mark.gpu
@@ -73,3 +74,59 @@ def test_attention_whole_and_in_units(ops, plain, heads, kv_heads, head_dim, pag
         assert torch.isinf(spoilt[end]).all()
         assert torch.equal(torch.cat((spoilt[:end], spoilt[end + 1:])), torch.cat((got[:end], got[end + 1:])))
     ops.check_errors()
+
+
+@pytest.mark.parametrize("name", ["B", "C"])      # heads of 32 and of 48 (the general kernel's)
+def test_decode_loops_with_and_without_graphs(tmp_path, name):
+    """Loops of decode steps whose positions pass several borders of units of 64 keys: the same tokens,
+    and behind them the same logits to the bit, whether the steps are replayed or launched one by one."""
+    from mlx_one_b200.cache import CacheManager
+    from mlx_one_b200.engine.loading import load_model
+    from mlx_one_b200.engine.runner import Runner, StepEntry
+
+    config, _, page = CONFIGS[name]
+    loaded = load_model(make_model_dir(name, tmp_path, dtype=torch.float32), "float32", DEVICE)
+    results = []
+    for graphs in (True, False):
+        cache = CacheManager(loaded.model.cache_needs, page_size=page, capacity_tokens=1024, max_requests=2,
+                             dtype=torch.float32, device=DEVICE)
+        runner = Runner(loaded.model, cache)
+        runner.use_graphs = graphs
+        last = []
+        for i, tokens in enumerate(prompts(config["vocab_size"], (100, 59), seed=21)):
+            cache.open(i)
+            last.append(int(runner.step([StepEntry(i, tokens, (len(tokens) - 1,))]).argmax()))
+        chosen = runner.decode_steps([StepEntry(i, [t]) for i, t in enumerate(last)], 170)
+        logits = runner.step([StepEntry(i, [t], (0,)) for i, t in enumerate(chosen[-1].tolist())])
+        loaded.model.ops.check_errors()
+        assert (runner.graph_replays > 160) == graphs
+        results.append((chosen.cpu(), logits.cpu().clone()))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("portions", [[1, 1], [1, 9]])
+def test_positions_behind_the_table(ops, portions):
+    """A host bound that the device's positions have outgrown changes nothing; a position behind the
+    block table raises the error flag, with the units of a token cut apart and with none cut."""
+    page, heads, kv_heads, dim = 16, 4, 2, 32
+    ctx, table, pages = make_batch(portions, [700, 63], page, DEVICE)
+    ctx.leading_single = 1 if portions[1] > 1 else 2
+    generator = torch.Generator(DEVICE).manual_seed(1)
+    kv = torch.randn(2, pages, kv_heads, page, dim, generator=generator, device=DEVICE)
+    q = torch.randn(ctx.tokens, heads, dim, generator=generator, device=DEVICE)
+    count, need = ops._sm_count, PagedKeyValues(kv_heads, dim, None)
+
+    def attend(table):
+        return ops.paged_attention(q, heads=heads, kv_heads=kv_heads, head_dim=dim, scale=0.2, window=None,
+                                   ctx=ctx, view=PagedView(kv, table, page, need))
+
+    try:
+        for ops._sm_count in (0, 1 << 30):
+            want, ctx.max_context = attend(table), 65
+            assert torch.equal(attend(table), want)
+            ops.check_errors()
+            attend(table[:, :40].contiguous())          # 640 keys, position 700
+            with pytest.raises(RuntimeError):
+                ops.check_errors()
+    finally:
+        ops._sm_count = count
