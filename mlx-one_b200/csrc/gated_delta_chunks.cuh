@@ -10,7 +10,8 @@
 // the 32 x 32 matrices T diag(beta) and P T diag(beta) with P(t, j) = D(t, j) (q_t . k_j), is worked out for
 // all chunks side by side; the walk over the chunks is then three products a chunk and five barriers
 // instead of a chain of sums and shuffles per four tokens. All in 32-bit; decays are multiplied up and
-// never divided, so a decay of zero is like any other.
+// never divided, so a decay of zero is like any other. What is not finite in a token reaches itself and
+// later tokens only: above the diagonals nothing is multiplied.
 #pragma once
 
 #include "delta_common.cuh"
@@ -185,7 +186,8 @@ delta_chunk_prepare_kernel(const float* q_in, const float* k_in, const float* co
         }
 #pragma unroll
         for (int t = 0; t < DC; ++t) {
-            column[t] *= beta;
+            // (above the diagonal by selection: a later token's beta may be NaN)
+            column[t] = lane <= t ? column[t] * beta : 0.f;
             out[t * DC + lane] = column[t];
         }
 #pragma unroll
@@ -221,9 +223,12 @@ constexpr int DC_BUFFER = 2 * DC * DC_PITCH + DC * DC_COLUMNS + 2 * DC * DC_SMAL
 constexpr size_t DC_WALK_SHARED =
     sizeof(float) * ((size_t)DC_BUFFERS * DC_BUFFER + DC_KEY * DC_COLUMNS + 8 * 2 * DC * DC_COLUMNS + 2 * DC * DC_COLUMNS);
 
-// part[warp][64][16] = x[64 rows, 4 STEPS columns from e0] * y[4 STEPS rows, 16 columns]
-template <int STEPS>
-__device__ __forceinline__ void chunk_product(const float* x, int pitch, const float* y, float* part) {
+// part[warp][64][16] = x[64 rows, 4 STEPS columns from e0] * y[4 STEPS rows, 16 columns]. LOWER: x is two
+// matrices of 32 rows that are zero above the diagonal (`column`: where its first column here stands), and
+// what stands there meets nothing of y.
+template <int STEPS, bool LOWER = false>
+__device__ __forceinline__ void chunk_product(const float* x, int pitch, const float* y, float* part,
+                                              int column = 0) {
     const int lane = threadIdx.x & 31, rg = lane >> 2, cg = lane & 3;
     FloatPair acc[8][2];
 #pragma unroll
@@ -237,14 +242,14 @@ __device__ __forceinline__ void chunk_product(const float* x, int pitch, const f
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const float4 v = *reinterpret_cast<const float4*>(x + (rg + 8 * i) * pitch + step * 4);
-            FloatPair f = pair_of(v.x);
-            fma_pair(acc[i][0], f, b[0].x); fma_pair(acc[i][1], f, b[0].y);
-            f = pair_of(v.y);
-            fma_pair(acc[i][0], f, b[1].x); fma_pair(acc[i][1], f, b[1].y);
-            f = pair_of(v.z);
-            fma_pair(acc[i][0], f, b[2].x); fma_pair(acc[i][1], f, b[2].y);
-            f = pair_of(v.w);
-            fma_pair(acc[i][0], f, b[3].x); fma_pair(acc[i][1], f, b[3].y);
+            const float values[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (LOWER && column + step * 4 + e > (rg + 8 * i) % DC) continue;
+                const FloatPair f = pair_of(values[e]);
+                fma_pair(acc[i][0], f, b[e].x);
+                fma_pair(acc[i][1], f, b[e].y);
+            }
         }
     }
 #pragma unroll
@@ -350,15 +355,21 @@ delta_walk_kernel(const float* q_in, const float* k_in, const float* v_in, const
         __syncthreads();
         float4 with_q = gather();                            // (rows of k: becomes r)
         const float before = decays[row % DC];
+        bool finite = true;
         if (row < DC) {
             const float4 v = *reinterpret_cast<const float4*>(vs + row * DC_COLUMNS + own_column);
-            *reinterpret_cast<float4*>(rest + row * DC_COLUMNS + own_column) =
-                make_float4(fmaf(-before, with_q.x, v.x), fmaf(-before, with_q.y, v.y),
-                            fmaf(-before, with_q.z, v.z), fmaf(-before, with_q.w, v.w));
+            const float4 r = make_float4(fmaf(-before, with_q.x, v.x), fmaf(-before, with_q.y, v.y),
+                                         fmaf(-before, with_q.z, v.z), fmaf(-before, with_q.w, v.w));
+            finite = isfinite(r.x) && isfinite(r.y) && isfinite(r.z) && isfinite(r.w);
+            *reinterpret_cast<float4*>(rest + row * DC_COLUMNS + own_column) = r;
         }
-        __syncthreads();
-        chunk_product<1>(small + warp * 4, DC_SMALL, rest + warp * 4 * DC_COLUMNS,
-                         part + warp * 2 * DC * DC_COLUMNS);
+        // (zero times an infinity or NaN of a later token would reach the tokens before it)
+        if (__syncthreads_and(finite))
+            chunk_product<1>(small + warp * 4, DC_SMALL, rest + warp * 4 * DC_COLUMNS,
+                             part + warp * 2 * DC * DC_COLUMNS);
+        else
+            chunk_product<1, true>(small + warp * 4, DC_SMALL, rest + warp * 4 * DC_COLUMNS,
+                                   part + warp * 2 * DC * DC_COLUMNS, warp * 4);
         __syncthreads();
         const float4 sum = gather();
         if (row < DC) {

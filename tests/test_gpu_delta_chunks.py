@@ -54,3 +54,37 @@ def test_portions_around_a_chunk(ops, dtype, heads, kv_heads, value_dim, steps, 
         # (the bounds of the recurrence's own test: 32-bit sums, 8 bits of mantissa at values of up to 8)
         assert difference < bound(dtype, 5e-5, 0.1), f"request {r}: {difference}"
     assert torch.isnan(state[[0, 2, 4]]).all() and torch.isfinite(state[[1, 3]]).all()
+
+
+@pytest.mark.parametrize("part", ["query", "key", "value", "gate", "beta", "decay"])
+@pytest.mark.parametrize("spoilt", [float("inf"), float("nan")])
+@pytest.mark.parametrize("at", [1, 37, 69])
+def test_what_is_not_finite_stays_behind_its_token(ops, part, spoilt, at):
+    """An infinity or NaN in one token of a portion of 70 (in the middle of a chunk of 32, near its start
+    and in the last, short one): the tokens before it keep their bits, other requests too."""
+    from mlx_one_b200.parts import FixedState, StateView
+    from mlx_one_b200.parts.mixers import GatedDeltaRule
+
+    H, G, D, V, taps = 4, 2, 128, 32, 4
+    sizes = dict(heads=H, kv_heads=G, key_dim=D, value_dim=V, taps=taps)
+    channels, inner = 2 * G * D + H * V, H * V
+    column = {"query": 5, "key": G * D + 5, "value": 2 * G * D + 5, "gate": channels + 5,
+              "beta": channels + inner, "decay": channels + inner + H}[part]
+    generator = torch.Generator(DEVICE).manual_seed(3)
+    normal = lambda *shape: torch.randn(shape, generator=generator, device=DEVICE)
+    rows = normal(70 + 40, channels + inner + 2 * H)
+    constants = dict(conv=0.5 * normal(channels, taps), a_log=normal(H) - 2, dt_bias=normal(H),
+                     norm_weight=1 + 0.2 * normal(V), eps=1e-5, unit_eps=1e-6, write=True, **sizes)
+    outputs = []
+    for value in (None, spoilt):
+        if value is not None:
+            rows[at, column] = value
+        size = GatedDeltaRule.state_size(sizes)
+        view = StateView(torch.zeros(2, size, device=DEVICE),
+                         torch.tensor([1, 0], dtype=torch.int32, device=DEVICE), FixedState((size,), "float32"))
+        outputs.append(ops.gated_delta_rule(rows, ctx=context([70, 40], [0, 0]), view=view, **constants))
+    ops.check_errors()
+    assert torch.isfinite(outputs[0]).all()
+    assert torch.equal(outputs[1][:at], outputs[0][:at]) and torch.equal(outputs[1][70:], outputs[0][70:])
+    if part in ("value", "key"):
+        assert not torch.isfinite(outputs[1][at]).all()
