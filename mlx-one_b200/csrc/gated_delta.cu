@@ -35,6 +35,8 @@
 #include "delta_common.cuh"
 #include "gated_delta_chunks.cuh"
 
+#include <algorithm>
+
 namespace {
 
 constexpr int PREP_THREADS = 256;
@@ -257,48 +259,47 @@ delta_prepare_runs_kernel(const T* projected, const float* __restrict__ conv, co
 }
 
 // ------------------------------------------------------------------ scan
-// Grid (column tiles, H + 1, requests); blocks with blockIdx.y == H write the convolution's
+// A block of THREADS threads: request r, head h and a tile of columns; h == H writes the convolution's
 // inputs into the ring. A thread keeps PER values of its column: element e of lane l is row
 // (e / 4) * 4 LANES + l * 4 + e % 4 of S, so that the lanes read k and q as neighbouring float4.
-// Dynamic shared memory: two buffers of [CHUNK][ROWS] for k and for q, [CHUNK][COLUMNS] for v and
-// [CHUNK] for each of g, beta and k.q.
-template <typename T, int PER, int LANES>
-__global__ void __launch_bounds__(SCAN_THREADS)
-delta_scan_kernel(const float* __restrict__ q_in, const float* __restrict__ k_in,
-                  const float* __restrict__ v_in, const float* __restrict__ coef,
-                  const float* __restrict__ kq, const T* __restrict__ projected,
-                  float* __restrict__ state, const int* __restrict__ slots,
-                  const int* __restrict__ request_start, const int* __restrict__ history,
-                  float* __restrict__ out, DeltaSizes sizes, int write, int ld) {
+// `staged`: two buffers of [CHUNK][ROWS] for k and for q, [CHUNK][COLUMNS] for v and [CHUNK] for each of g,
+// beta and k.q. A column's sums do not depend on THREADS.
+template <int PER, int LANES, int THREADS>
+constexpr size_t scan_shared() {
+    return (size_t)2 * CHUNK * (2 * PER * LANES + THREADS / LANES + 3) * sizeof(float);
+}
+
+template <typename T, int PER, int LANES, int THREADS>
+__device__ __forceinline__ void scan_portion(const float* q_in, const float* k_in, const float* v_in,
+                                             const float* coef, const float* kq, const T* projected,
+                                             float* state, const int* slots, int first, int last,
+                                             const int* history, float* out, const DeltaSizes& sizes,
+                                             int write, int ld, float* staged, int tile, int tiles, int h,
+                                             int r) {
     constexpr int ROWS = PER * LANES;                 // rows of S a thread group covers (>= D)
-    constexpr int COLUMNS = SCAN_THREADS / LANES;     // columns of S per block
+    constexpr int COLUMNS = THREADS / LANES;          // columns of S per block
     constexpr int BUFFER = CHUNK * (2 * ROWS + COLUMNS + 3);
     constexpr int GROUP = 4;                          // tokens worked on together
-    extern __shared__ __align__(16) float staged[];
     __shared__ float gram[CHUNK / GROUP][2][GROUP][GROUP];   // k_i.k_t and k_i.q_t, i < t in a group
-    griddep_wait();
-    const int r = blockIdx.z;
-    const int first = request_start[r], last = request_start[r + 1];
     const int H = sizes.heads, G = sizes.kv_heads, D = sizes.key_dim, V = sizes.value_dim;
     float* slot = state + (size_t)slots[r] * sizes.state();
-    if (blockIdx.y == H) {
+    if (h == H) {
         // the inputs of the portion's last positions (at most taps of them) go into the ring
         griddep_launch();
         if (!write) return;
         const int channels = sizes.channels(), taps = sizes.taps;
         const int n = last - first, kept = min(n, taps);
         float* ring = slot + sizes.matrices();
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < channels;
-             c += gridDim.x * blockDim.x)
+        for (int c = tile * THREADS + threadIdx.x; c < channels; c += tiles * THREADS)
             for (int index = n - kept; index < n; ++index)
                 ring[(size_t)((history[r] + index) % taps) * channels + c] =
                     to_float<T>(projected[(size_t)(first + index) * ld + c]);
         return;
     }
-    const int h = blockIdx.y, g = h / (H / G);
+    const int g = h / (H / G);
     const int lane = threadIdx.x & (LANES - 1);
     const int local = threadIdx.x / LANES;
-    const int column = blockIdx.x * COLUMNS + local;
+    const int column = tile * COLUMNS + local;
     const bool live = column < V;
     float* matrix = slot + (size_t)h * D * V;
     float S[PER];
@@ -312,7 +313,7 @@ delta_scan_kernel(const float* __restrict__ q_in, const float* __restrict__ k_in
                        ((reinterpret_cast<uintptr_t>(q_in) | reinterpret_cast<uintptr_t>(k_in) |
                          reinterpret_cast<uintptr_t>(v_in)) & 15) == 0;
     // rows behind D and columns behind V stay zero in both buffers
-    for (int i = threadIdx.x; i < 2 * BUFFER; i += SCAN_THREADS) staged[i] = 0.f;
+    for (int i = threadIdx.x; i < 2 * BUFFER; i += THREADS) staged[i] = 0.f;
     __syncthreads();
     auto fetch = [&](int base, int buffer) {
         const int count = min(CHUNK, last - base);
@@ -320,35 +321,35 @@ delta_scan_kernel(const float* __restrict__ q_in, const float* __restrict__ k_in
         float* qs = ks + CHUNK * ROWS;
         float* vs = qs + CHUNK * ROWS;
         float* cs = vs + CHUNK * COLUMNS;
-        const int wide = min(COLUMNS, V - (int)blockIdx.x * COLUMNS);
+        const int wide = min(COLUMNS, V - tile * COLUMNS);
         if (quads) {
             // rows of a multiple of four values: 16 bytes a copy
             const int per_row = D / 4;
             const bool power = (per_row & (per_row - 1)) == 0;
             const int shift = __ffs(per_row) - 1;
-            for (int i = threadIdx.x; i < count * per_row; i += SCAN_THREADS) {
+            for (int i = threadIdx.x; i < count * per_row; i += THREADS) {
                 const int t = power ? i >> shift : i / per_row;
                 const int e = (i - t * per_row) * 4;
                 const size_t at = ((size_t)(base + t) * G + g) * D + e;
                 copy_async_16(ks + t * ROWS + e, k_in + at);
                 copy_async_16(qs + t * ROWS + e, q_in + at);
             }
-            for (int i = threadIdx.x; i < count * (wide / 4); i += SCAN_THREADS) {
+            for (int i = threadIdx.x; i < count * (wide / 4); i += THREADS) {
                 const int t = i / (wide / 4), c = (i % (wide / 4)) * 4;
                 copy_async_16(vs + t * COLUMNS + c,
-                              v_in + ((size_t)(base + t) * H + h) * V + blockIdx.x * COLUMNS + c);
+                              v_in + ((size_t)(base + t) * H + h) * V + tile * COLUMNS + c);
             }
         } else {
-            for (int i = threadIdx.x; i < count * D; i += SCAN_THREADS) {
+            for (int i = threadIdx.x; i < count * D; i += THREADS) {
                 const int t = i / D, e = i % D;
                 const size_t at = ((size_t)(base + t) * G + g) * D + e;
                 copy_async_4(ks + t * ROWS + e, k_in + at);
                 copy_async_4(qs + t * ROWS + e, q_in + at);
             }
-            for (int i = threadIdx.x; i < count * wide; i += SCAN_THREADS) {
+            for (int i = threadIdx.x; i < count * wide; i += THREADS) {
                 const int t = i / wide, c = i % wide;
                 copy_async_4(vs + t * COLUMNS + c,
-                             v_in + ((size_t)(base + t) * H + h) * V + blockIdx.x * COLUMNS + c);
+                             v_in + ((size_t)(base + t) * H + h) * V + tile * COLUMNS + c);
             }
         }
         if (threadIdx.x < count) {
@@ -381,7 +382,7 @@ delta_scan_kernel(const float* __restrict__ q_in, const float* __restrict__ k_in
         const float* cs = vs + CHUNK * COLUMNS;
         // the products k_i.k_t and k_i.q_t of the pairs i < t inside each group of four tokens:
         // 4 groups x 6 pairs x 2 kinds, each by LANES lanes
-        for (int item = threadIdx.x / LANES; item < (CHUNK / GROUP) * 12; item += SCAN_THREADS / LANES) {
+        for (int item = threadIdx.x / LANES; item < (CHUNK / GROUP) * 12; item += THREADS / LANES) {
             const int group = item / 12, kind = (item % 12) / 6, pair = item % 6;
             const int t = pair < 1 ? 1 : (pair < 3 ? 2 : 3);
             const int i = pair - (t == 1 ? 0 : (t == 2 ? 1 : 3));
@@ -483,6 +484,55 @@ delta_scan_kernel(const float* __restrict__ q_in, const float* __restrict__ k_in
             const int row = (e / 4) * (4 * LANES) + lane * 4 + e % 4;
             if (row < D) matrix[(size_t)row * V + column] = S[e];
         }
+    }
+}
+
+// Grid (column tiles, H + 1, requests).
+template <typename T, int PER, int LANES>
+__global__ void __launch_bounds__(SCAN_THREADS)
+delta_scan_kernel(const float* __restrict__ q_in, const float* __restrict__ k_in,
+                  const float* __restrict__ v_in, const float* __restrict__ coef,
+                  const float* __restrict__ kq, const T* __restrict__ projected,
+                  float* __restrict__ state, const int* __restrict__ slots,
+                  const int* __restrict__ request_start, const int* __restrict__ history,
+                  float* __restrict__ out, DeltaSizes sizes, int write, int ld) {
+    extern __shared__ __align__(16) float staged[];
+    griddep_wait();
+    const int r = blockIdx.z;
+    scan_portion<T, PER, LANES, SCAN_THREADS>(q_in, k_in, v_in, coef, kq, projected, state, slots,
+                                              request_start[r], request_start[r + 1], history, out, sizes,
+                                              write, ld, staged, blockIdx.x, gridDim.x, blockIdx.y, r);
+}
+
+// The first of the two kernels of steps with portions of `chunk_from` tokens and more. Grid (places and more,
+// query/key heads): the blocks of the first `places` prepare the chunks of those portions, the others, where
+// there may be shorter portions (SHORTER), scan these (column tiles x (H + 1) x requests); neither needs the
+// other.
+template <typename T, bool SHORTER>
+__global__ void __launch_bounds__(DC_THREADS, 2)
+delta_chunk_prepare_kernel(const float* q_in, const float* k_in, const float* v_in, const float* coef,
+                           const float* kq, const T* projected, float* state, const int* __restrict__ slots,
+                           const int* __restrict__ request_start, const int* __restrict__ history,
+                           float* out, float* chunks, DeltaSizes sizes, int requests, int lead,
+                           int chunk_from, int places, int write, int ld) {
+    constexpr int COLUMNS = DC_THREADS / 8;
+    extern __shared__ __align__(16) float shared[];
+    griddep_wait();
+    griddep_launch();
+    if (!SHORTER || (int)blockIdx.x < places) {
+        prepare_chunk(q_in, k_in, coef, request_start, chunks, sizes, requests, lead, chunk_from, shared);
+        return;
+    }
+    if constexpr (SHORTER) {
+        const int tiles = (sizes.value_dim + COLUMNS - 1) / COLUMNS;
+        const int item = (blockIdx.x - places) * gridDim.y + blockIdx.y;
+        const int tile = item % tiles, h = item / tiles % (sizes.heads + 1), r = item / tiles / (sizes.heads + 1);
+        if (r >= requests) return;
+        const int first = request_start[r], last = request_start[r + 1];
+        if (last - first >= chunk_from) return;
+        scan_portion<T, DC_KEY / 8, 8, DC_THREADS>(q_in, k_in, v_in, coef, kq, projected, state, slots, first,
+                                                   last, history, out, sizes, write, ld, shared, tile, tiles, h,
+                                                   r);
     }
 }
 
@@ -680,19 +730,20 @@ delta_finish_kernel(const float* __restrict__ o, const T* __restrict__ projected
         mixed[item * V + e] = from_float<T>(row[e] * inv * weight[e] * silu(to_float<T>(gate[e])));
 }
 
-// (scratch and state are allocations of their own, so rows of q, k and v are aligned to 16 bytes)
-bool delta_in_chunks(int tokens, int requests, const DeltaSizes& sizes) {
-    return sizes.key_dim == DC_KEY && sizes.value_dim % DC_COLUMNS == 0 && tokens >= 8 * requests;
+// Whether a step with portions of up to `longest` tokens has some that are worked on in chunks. (Scratch
+// and state are allocations of their own, so rows of q, k and v are aligned to 16 bytes.)
+bool delta_in_chunks(int longest, int chunk_from, const DeltaSizes& sizes) {
+    return sizes.key_dim == DC_KEY && sizes.value_dim % DC_COLUMNS == 0 && longest >= chunk_from;
 }
 
 template <typename T>
 int launch_delta(const void* projected, const float* conv, const float* a_log, const float* dt_bias,
                  const float* norm_weight, float eps, float unit_eps, float* state,
                  const int* slots, const int* token_request, const int* request_start,
-                 const int* history, float* scratch, void* mixed, int tokens, int requests,
-                 DeltaSizes sizes, int write, int ld, int single, cudaStream_t stream) {
+                 const int* history, float* scratch, void* mixed, int tokens, int requests, int longest,
+                 int lead, int chunk_from, DeltaSizes sizes, int write, int ld, cudaStream_t stream) {
     const int G = sizes.kv_heads, D = sizes.key_dim, H = sizes.heads, V = sizes.value_dim;
-    if (single && tokens == requests && V <= STEP_MAX_COLUMNS) {
+    if (longest == 1 && tokens == requests && V <= STEP_MAX_COLUMNS) {
         // every request brings one token: one kernel
         const int per = D <= 16 ? 4 : D <= 32 ? 8 : D <= 64 ? 16 : D <= 128 ? 32 : 64;
         const size_t shared = (size_t)(2 * per * STEP_LANES + 2 * V) * sizeof(float);
@@ -739,49 +790,57 @@ int launch_delta(const void* projected, const float* conv, const float* a_log, c
                       token_request, request_start, history, q, k, v, coef, kq, sizes, unit_eps, ld);
     }
     MLXONE_LAUNCH_CHECK("gated delta rule (prepare)");
-    // Keys of 128 values and portions of some length: 32 tokens at a time. A chunk takes the walk about
-    // as long as eight tokens take the scan below, so below eight tokens a request the scan is ahead.
+    // Keys of 128 values: portions of `chunk_from` tokens and more 32 tokens at a time, shorter ones beside
+    // them. A portion's own length decides and nothing else of the step, so that a request's results do not
+    // depend on its neighbours.
     float* chunks = kq + (size_t)tokens * G;
     chunks += (4 - (chunks - scratch) % 4) % 4;
-    if (delta_in_chunks(tokens, requests, sizes)) {
-        cudaFuncSetAttribute(delta_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)DC_PREPARE_SHARED);
+    if (delta_in_chunks(longest, chunk_from, sizes)) {
+        const bool shorter = requests > 1 || tokens < chunk_from;
+        auto prepare = shorter ? delta_chunk_prepare_kernel<T, true> : delta_chunk_prepare_kernel<T, false>;
+        const size_t shared = std::max(DC_PREPARE_SHARED, scan_shared<DC_KEY / 8, 8, DC_THREADS>());
+        cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
         cudaFuncSetAttribute(delta_walk_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)DC_WALK_SHARED);
-        launch_kernel(delta_chunk_prepare_kernel, dim3(chunk_places(tokens, requests), G), dim3(DC_THREADS),
-                      DC_PREPARE_SHARED, stream, true, (const float*)q, (const float*)k, (const float*)coef,
-                      request_start, chunks, sizes, requests);
+        // (the first `lead` requests are known to bring one token each)
+        const int places = chunk_places(tokens - lead, requests - lead);
+        const long long scans = shorter ? (long long)ceil_div_host(V, DC_THREADS / 8) * (H + 1) * requests : 0;
+        MLXONE_REQUIRE(scans <= 0x7fffffffLL - G, "gated delta rule: too many requests");
+        launch_kernel(prepare, dim3(places + ceil_div_host(scans, G), G), dim3(DC_THREADS), shared, stream,
+                      true, (const float*)q, (const float*)k, (const float*)v, (const float*)coef,
+                      (const float*)kq, (const T*)projected, state, slots, request_start, history, o, chunks,
+                      sizes, requests, lead, chunk_from, places, write, ld);
         MLXONE_LAUNCH_CHECK("gated delta rule (chunks)");
-        launch_kernel(delta_walk_kernel<T>, dim3(V / DC_COLUMNS, H + 1, requests), dim3(DC_THREADS),
+        launch_kernel(delta_walk_kernel<T>, dim3(V / DC_COLUMNS, H + 1, requests - lead), dim3(DC_THREADS),
                       DC_WALK_SHARED, stream, true, (const float*)q, (const float*)k, (const float*)v,
                       (const float*)chunks, (const T*)projected, state, slots, request_start, history, o,
-                      sizes, write, ld);
+                      sizes, lead, chunk_from, write, ld);
         MLXONE_LAUNCH_CHECK("gated delta rule (walk)");
     } else {
-    // A column's values are spread over 8 lanes (16 for keys longer than 128). Measured at 16 heads
-    // of 128 x 128 and 2048 tokens: with 16 lanes every lane repeats the four tokens' solve for
-    // half as many values of its own, 292 M warp instructions and 702 us.
-#define SCAN(PER, LANES)                                                                          \
-    do {                                                                                          \
-        constexpr int COLUMNS = SCAN_THREADS / LANES;                                             \
-        const dim3 grid(ceil_div_host(V, COLUMNS), H + 1, requests);                              \
-        const size_t staged = (size_t)2 * CHUNK * (2 * PER * LANES + COLUMNS + 3) * sizeof(float); \
-        if (staged > 48 * 1024)                                                                   \
-            cudaFuncSetAttribute(delta_scan_kernel<T, PER, LANES>,                                \
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staged);       \
-        launch_kernel(delta_scan_kernel<T, PER, LANES>, grid, dim3(SCAN_THREADS), staged, stream, \
-                      true, (const float*)q, (const float*)k, (const float*)v,                    \
-                      (const float*)coef, (const float*)kq, (const T*)projected, state, slots,    \
-                      request_start, history, o, sizes, write, ld);                               \
-    } while (0)
-    // ... with 8 lanes 156 M instructions and 536 us. (16 lanes only where a grid of 8-lane blocks
-    // would leave half the SMs empty was measured too, 8 heads: 1112 us against 947 us.)
-    if (D <= 32) SCAN(4, 8);
-    else if (D <= 64) SCAN(8, 8);
-    else if (D <= 128) SCAN(16, 8);
-    else SCAN(16, 16);
+        // A column's values are spread over 8 lanes (16 for keys longer than 128). Measured at 16 heads
+        // of 128 x 128 and 2048 tokens: with 16 lanes every lane repeats the four tokens' solve for
+        // half as many values of its own, 292 M warp instructions and 702 us.
+#define SCAN(PER, LANES)                                                                              \
+        do {                                                                                          \
+            constexpr int COLUMNS = SCAN_THREADS / LANES;                                             \
+            const dim3 grid(ceil_div_host(V, COLUMNS), H + 1, requests);                              \
+            const size_t staged = scan_shared<PER, LANES, SCAN_THREADS>();\
+            if (staged > 48 * 1024)                                                                   \
+                cudaFuncSetAttribute(delta_scan_kernel<T, PER, LANES>,                                \
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staged);       \
+            launch_kernel(delta_scan_kernel<T, PER, LANES>, grid, dim3(SCAN_THREADS), staged, stream, \
+                          true, (const float*)q, (const float*)k, (const float*)v,                    \
+                          (const float*)coef, (const float*)kq, (const T*)projected, state, slots,    \
+                          request_start, history, o, sizes, write, ld);                               \
+        } while (0)
+        // ... with 8 lanes 156 M instructions and 536 us. (16 lanes only where a grid of 8-lane blocks
+        // would leave half the SMs empty was measured too, 8 heads: 1112 us against 947 us.)
+        if (D <= 32) SCAN(4, 8);
+        else if (D <= 64) SCAN(8, 8);
+        else if (D <= 128) SCAN(16, 8);
+        else SCAN(16, 16);
 #undef SCAN
-    MLXONE_LAUNCH_CHECK("gated delta rule (scan)");
+        MLXONE_LAUNCH_CHECK("gated delta rule (scan)");
     }
     const long long items = (long long)tokens * H;
     launch_kernel(delta_finish_kernel<T>, dim3(ceil_div_host(items, 8)), dim3(256), 0, stream, true,
@@ -794,19 +853,21 @@ int launch_delta(const void* projected, const float* conv, const float* a_log, c
 
 }  // namespace
 
-MLXONE_API int mlxone_gated_delta_in_chunks(int tokens, int requests, int heads, int kv_heads, int key_dim,
-                                            int value_dim) {
-    return delta_in_chunks(tokens, requests, {heads, kv_heads, key_dim, value_dim, 1});
+// Kernels that a step with portions takes (arguments: see mlxone_gated_delta).
+MLXONE_API int mlxone_gated_delta_launches(int longest, int chunk_from, int heads, int kv_heads, int key_dim,
+                                           int value_dim) {
+    return delta_in_chunks(longest, chunk_from, {heads, kv_heads, key_dim, value_dim, 1}) ? 4 : 3;
 }
 
-// 32-bit values of scratch that a call with `tokens` tokens needs.
-MLXONE_API long long mlxone_gated_delta_scratch(int tokens, int requests, int heads, int kv_heads,
-                                                int key_dim, int value_dim) {
+// 32-bit values of scratch that a call with `tokens` tokens needs (arguments: see mlxone_gated_delta).
+MLXONE_API long long mlxone_gated_delta_scratch(int tokens, int requests, int longest, int lead,
+                                                int chunk_from, int heads, int kv_heads, int key_dim,
+                                                int value_dim) {
     const DeltaSizes sizes = {heads, kv_heads, key_dim, value_dim, 1};
     const long long rows = (long long)tokens * (2LL * kv_heads * key_dim + 2LL * heads * value_dim +
                                                 2LL * heads + kv_heads);
-    if (!delta_in_chunks(tokens, requests, sizes)) return rows;
-    return rows + 4 + (long long)chunk_places(tokens, requests) * heads * DC_VALUES;
+    if (!delta_in_chunks(longest, chunk_from, sizes)) return rows;
+    return rows + 4 + (long long)chunk_places(tokens - lead, requests - lead) * heads * DC_VALUES;
 }
 
 // 32-bit values of a request's slot.
@@ -816,14 +877,17 @@ MLXONE_API long long mlxone_gated_delta_state(int heads, int kv_heads, int key_d
     return sizes.state();
 }
 
+// `longest`: a bound of the tokens that a request brings, 1 only if every request brings one. `lead`: how
+// many requests at the head of the step are known to bring one token each (0 is always right). `chunk_from`:
+// portions of that many tokens and more are worked on in chunks, where keys have 128 values.
 MLXONE_API int mlxone_gated_delta(const void* projected, const float* conv, const float* a_log,
                                   const float* dt_bias, const float* norm_weight, float eps,
                                   float unit_eps, float* state, const int* slots,
                                   const int* token_request, const int* request_start,
                                   const int* history, float* scratch, void* mixed, int tokens,
-                                  int requests, int heads, int kv_heads, int key_dim, int value_dim,
-                                  int taps, int write, int ld, int single, int dtype,
-                                  cudaStream_t stream) {
+                                  int requests, int longest, int lead, int chunk_from, int heads,
+                                  int kv_heads, int key_dim, int value_dim, int taps, int write, int ld,
+                                  int dtype, cudaStream_t stream) {
     if (tokens == 0) return 0;
     MLXONE_REQUIRE(tokens > 0 && requests > 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0,
                    "gated delta rule: bad sizes");
@@ -831,15 +895,18 @@ MLXONE_API int mlxone_gated_delta(const void* projected, const float* conv, cons
                    key_dim);
     MLXONE_REQUIRE(value_dim >= 1 && taps >= 1, "gated delta rule: bad value size or taps");
     MLXONE_REQUIRE(requests <= 65535 && heads < 65535, "gated delta rule: too many requests or heads");
+    MLXONE_REQUIRE(longest >= 1 && chunk_from >= 1 && lead >= 0 && lead <= requests && lead <= tokens &&
+                       (lead < requests || longest == 1),
+                   "gated delta rule: %d of %d requests cannot bring one token each", lead, requests);
     const DeltaSizes sizes = {heads, kv_heads, key_dim, value_dim, taps};
     MLXONE_REQUIRE(ld >= gated_width(sizes), "gated delta rule: rows %d apart are shorter than %d", ld,
                    gated_width(sizes));
     if (dtype == MLXONE_BF16)
         return launch_delta<__nv_bfloat16>(projected, conv, a_log, dt_bias, norm_weight, eps,
                                            unit_eps, state, slots, token_request, request_start,
-                                           history, scratch, mixed, tokens, requests, sizes, write,
-                                           ld, single, stream);
+                                           history, scratch, mixed, tokens, requests, longest, lead,
+                                           chunk_from, sizes, write, ld, stream);
     return launch_delta<float>(projected, conv, a_log, dt_bias, norm_weight, eps, unit_eps, state,
                                slots, token_request, request_start, history, scratch, mixed, tokens,
-                               requests, sizes, write, ld, single, stream);
+                               requests, longest, lead, chunk_from, sizes, write, ld, stream);
 }

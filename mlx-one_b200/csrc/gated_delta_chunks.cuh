@@ -26,9 +26,12 @@ constexpr int DC_THREADS = 256;
 // what a chunk and head leave for the walk: T diag(beta), P T diag(beta), G_t, D(32, t)
 constexpr int DC_VALUES = 2 * DC * DC + 2 * DC;
 
-// Requests' chunks lie one behind another; every request may leave one place unused.
+// Requests' chunks lie one behind another; every request may leave one place unused, and those of fewer than
+// `chunk_from` tokens leave theirs. The first `lead` requests, of one token each, have none.
 __host__ __device__ __forceinline__ int chunk_places(int tokens, int requests) { return tokens / DC + requests; }
-__device__ __forceinline__ int first_chunk(int first_token, int request) { return first_token / DC + request; }
+__device__ __forceinline__ int first_chunk(int first_token, int request, int lead) {
+    return (first_token - lead) / DC + request - lead;
+}
 
 // 16 bytes, or zeros
 __device__ __forceinline__ void copy_or_zero_16(float* dst, const float* src, bool live) {
@@ -64,7 +67,8 @@ __device__ __forceinline__ float4 quad_of(FloatPair a, FloatPair b) {
 }
 
 // ------------------------------------------------------------------ what does not need S
-// Grid (chunk places, query/key heads). The products of the chunk's k and q with its k: a warp takes 16
+// One block of DC_THREADS threads per place of a chunk (x) and query/key head (y) (`shared`: DC_PREPARE_SHARED
+// bytes). The products of the chunk's k and q with its k: a warp takes 16
 // of the 128 values of a key, a lane 8 x 8 products (16 values read from shared memory for 64 FMAs:
 // shared memory gives a thread's value for every four FMAs that an SM can do); then a warp per value
 // head, lane = column: T by forward substitution in registers, P T behind it. (A and P of up to three
@@ -74,11 +78,10 @@ constexpr int DC_SOLVERS = 3;
 constexpr size_t DC_PREPARE_SHARED = sizeof(float) * ((size_t)2 * DC * DC_PITCH + 8 * 2 * DC * DC);
 static_assert(DC_SOLVERS * 2 * DC * DC_SMALL <= 2 * DC * DC_PITCH, "A and P fit where k and q were");
 
-__global__ void __launch_bounds__(DC_THREADS, 2)
-delta_chunk_prepare_kernel(const float* q_in, const float* k_in, const float* coef,
-                           const int* __restrict__ request_start, float* chunks, DeltaSizes sizes,
-                           int requests) {
-    extern __shared__ __align__(16) float shared[];
+__device__ __forceinline__ void prepare_chunk(const float* q_in, const float* k_in, const float* coef,
+                                              const int* request_start, float* chunks,
+                                              const DeltaSizes& sizes, int requests, int lead,
+                                              int chunk_from, float* shared) {
     float* kq = shared;                                      // [k of 32 tokens, q of 32][DC_PITCH]
     float* part = kq + 2 * DC * DC_PITCH;                    // [8][64][32]
     __shared__ int place[2];                                 // first token, tokens
@@ -86,12 +89,10 @@ delta_chunk_prepare_kernel(const float* q_in, const float* k_in, const float* co
     const int H = sizes.heads, G = sizes.kv_heads, per_group = H / G;
     if (tid == 0) place[1] = 0;
     __syncthreads();
-    griddep_wait();
-    griddep_launch();
-    for (int r = tid; r < requests; r += DC_THREADS) {
+    for (int r = lead + tid; r < requests; r += DC_THREADS) {
         const int first = request_start[r], count = request_start[r + 1] - first;
-        const int c = (int)blockIdx.x - first_chunk(first, r);
-        if (c >= 0 && c * DC < count) {
+        const int c = (int)blockIdx.x - first_chunk(first, r, lead);
+        if (count >= chunk_from && c >= 0 && c * DC < count) {
             place[0] = first + c * DC;
             place[1] = min(DC, count - c * DC);
         }
@@ -210,8 +211,8 @@ delta_chunk_prepare_kernel(const float* q_in, const float* k_in, const float* co
 }
 
 // ------------------------------------------------------------------ the walk
-// Grid (tiles of 16 columns of S, heads + 1, requests); blocks with blockIdx.y == heads write the
-// convolution's inputs into the ring. S lies in shared memory (and in the registers of the 128 threads
+// Grid (tiles of 16 columns of S, heads + 1, requests behind the first `lead`), of which those of fewer than
+// `chunk_from` tokens are the scan's; blocks with blockIdx.y == heads write the convolution's inputs into the ring. S lies in shared memory (and in the registers of the 128 threads
 // that update it). [k; q] S and [T diag(beta); P T diag(beta)] r are products of 64 rows by 16 columns: a
 // lane takes 8 x 4 outputs, a warp an eighth of the sum (16 values of a key, 4 tokens), and the eighths
 // are added up in order. Bound by the chain of products, barriers and reads of shared memory of a chunk
@@ -262,15 +263,16 @@ __global__ void __launch_bounds__(DC_THREADS)
 delta_walk_kernel(const float* q_in, const float* k_in, const float* v_in, const float* chunks,
                   const T* __restrict__ projected, float* state, const int* __restrict__ slots,
                   const int* __restrict__ request_start, const int* __restrict__ history, float* out,
-                  DeltaSizes sizes, int write, int ld) {
+                  DeltaSizes sizes, int lead, int chunk_from, int write, int ld) {
     extern __shared__ __align__(16) float shared[];
     float* matrix_s = shared + DC_BUFFERS * DC_BUFFER;       // S [128][16]
     float* part = matrix_s + DC_KEY * DC_COLUMNS;            // [8][64][16]
     float* rest = part + 8 * 2 * DC * DC_COLUMNS;            // r [32][16]
     float* moved = rest + DC * DC_COLUMNS;                   // D(32, t) u_t [32][16]
-    const int tid = threadIdx.x, warp = tid >> 5, r = blockIdx.z;
+    const int tid = threadIdx.x, warp = tid >> 5, r = lead + blockIdx.z;
     griddep_wait();
     const int first = request_start[r], last = request_start[r + 1];
+    if (last - first < chunk_from) return;
     const int H = sizes.heads, G = sizes.kv_heads, V = sizes.value_dim;
     float* slot = state + (size_t)slots[r] * sizes.state();
     if ((int)blockIdx.y == H) {
@@ -305,7 +307,7 @@ delta_walk_kernel(const float* q_in, const float* k_in, const float* v_in, const
                             v_in + ((size_t)(base + min(t, count - 1)) * H + h) * V + column0 + c, t < count);
         }
         to += DC * DC_COLUMNS;
-        const float* from = chunks + ((size_t)(first_chunk(first, r) + chunk) * H + h) * DC_VALUES;
+        const float* from = chunks + ((size_t)(first_chunk(first, r, lead) + chunk) * H + h) * DC_VALUES;
         for (int i = me; i < 2 * DC * (DC / 4); i += count_of) {
             const int row = i / (DC / 4), e = i % (DC / 4) * 4;
             copy_or_zero_16(to + row * DC_SMALL + e, from + row * DC + e, true);

@@ -117,6 +117,12 @@ class CudaOps:
         self.skinny_fused_max_rows = 16
         # latent attention of few tokens: the key up-projection with the queries' rotation in one kernel
         self.fused_latent = True
+        # The delta rule with keys of 128 values: portions from this length on are worked on in chunks of
+        # 32 tokens, shorter ones four tokens at a time. Microseconds a layer by chunks / by fours, 16
+        # heads of 128 x 128: one portion of 32 / 48 / 64 / 333 tokens 25 / 20, 27 / 24, 28 / 29, 53 /
+        # 100; four of 64 tokens 54 / 50; 16 of 32 / 48 / 64 tokens 93 / 88, 139 / 121, 145 / 155. 8 heads:
+        # 64 portions of 32 tokens 183 / 166; 16 of 64 82 / 87.
+        self.delta_chunk_from = 64
         # the gated recurrence of few single tokens: the gates' product in the recurrence's kernel
         self.fused_recurrence = True
         self._sample_scratch: torch.Tensor | None = None
@@ -1275,7 +1281,10 @@ class CudaOps:
             raise KernelError(f"a state slot has {view.state[0].numel()} values, the mixer needs {size}")
         # a step of single tokens runs as one kernel, else preparation, scan and finish
         single = ctx.max_portion == 1 and tokens == ctx.requests
-        scratch = torch.empty(self.lib.mlxone_gated_delta_scratch(tokens, ctx.requests, heads,
+        lead = min(getattr(ctx, "leading_single", 0), ctx.requests)
+        scratch = torch.empty(self.lib.mlxone_gated_delta_scratch(tokens, ctx.requests,
+                                                                  ctx.max_portion, lead,
+                                                                  self.delta_chunk_from, heads,
                                                                   kv_heads, key_dim, value_dim),
                               dtype=torch.float32, device=self.device)
         out = torch.empty((tokens, inner), dtype=projected.dtype, device=self.device)
@@ -1285,14 +1294,14 @@ class CudaOps:
                    _c_void_p(_ptr(view.slots)), _c_void_p(_ptr(ctx.token_request)),
                    _c_void_p(_ptr(ctx.request_start)), _c_void_p(_ptr(ctx.history)),
                    _c_void_p(_ptr(scratch)), _c_void_p(_ptr(out)), _c_int(tokens),
-                   _c_int(ctx.requests), _c_int(heads), _c_int(kv_heads), _c_int(key_dim),
+                   _c_int(ctx.requests), _c_int(ctx.max_portion), _c_int(lead),
+                   _c_int(self.delta_chunk_from), _c_int(heads), _c_int(kv_heads), _c_int(key_dim),
                    _c_int(value_dim), _c_int(taps), _c_int(1 if write else 0),
-                   _c_int(projected.stride(0)), _c_int(1 if single else 0),
-                   _c_int(_dtype_code(projected.dtype)))
+                   _c_int(projected.stride(0)), _c_int(_dtype_code(projected.dtype)))
         if not (single and value_dim <= 128):
             # preparation, scan and finish; chunks of long portions have a kernel more
-            self.launches += 2 + self.lib.mlxone_gated_delta_in_chunks(
-                tokens, ctx.requests, heads, kv_heads, key_dim, value_dim)
+            self.launches += self.lib.mlxone_gated_delta_launches(
+                ctx.max_portion, self.delta_chunk_from, heads, kv_heads, key_dim, value_dim) - 1
         return out
 
     def channel_delta_rule(self, projected, decay_up, gate_up, *, decay_columns, gate_columns, conv,

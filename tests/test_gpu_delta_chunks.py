@@ -9,9 +9,17 @@ from test_gpu_galarax import DEVICE, DTYPES, bound, context, delta_pieces, ops  
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def short_portions_in_chunks_too(ops):
+    kept, ops.delta_chunk_from = ops.delta_chunk_from, 8
+    yield
+    ops.delta_chunk_from = kept
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads, kv_heads, value_dim", [(2, 1, 16), (3, 3, 48), (20, 2, 32)])
-@pytest.mark.parametrize("steps", [[(32, 40)], [(33, 31)], [(64, 1), (95, 65)], [(1, 70), (127, 3), (1, 30)]])
+@pytest.mark.parametrize("steps", [[(32, 40)], [(33, 31)], [(64, 1), (95, 65)], [(1, 70), (127, 3), (1, 30)],
+                                   [(40, 30), (7, 8), (8, 8)]])
 @pytest.mark.parametrize("forget", [-5.0, 5.0])
 def test_portions_around_a_chunk(ops, dtype, heads, kv_heads, value_dim, steps, forget):
     """``forget``: log of the decay's rate; at 5 most decays are zero in 32-bit."""
@@ -88,3 +96,37 @@ def test_what_is_not_finite_stays_behind_its_token(ops, part, spoilt, at):
     assert torch.equal(outputs[1][:at], outputs[0][:at]) and torch.equal(outputs[1][70:], outputs[0][70:])
     if part in ("value", "key"):
         assert not torch.isfinite(outputs[1][at]).all()
+
+
+@pytest.mark.parametrize("portion", [1, 5, 7, 8, 40, 63, 64])
+@pytest.mark.parametrize("chunk_from", [8, 64])
+@pytest.mark.parametrize("beside, lead", [([1] * 30, 30), ([1] * 30, 4), ([2, 3], 0), ([100], 0), ([7, 300, 1], 0)])
+def test_a_portion_does_not_depend_on_its_neighbours(ops, portion, chunk_from, beside, lead):
+    """A request's portion by itself and behind others of all kinds (the first ``lead`` of them known to
+    bring one token): the same output and the same state, bit for bit."""
+    ops.delta_chunk_from = chunk_from
+    from mlx_one_b200.parts import FixedState, StateView
+    from mlx_one_b200.parts.mixers import GatedDeltaRule
+
+    sizes = dict(heads=4, kv_heads=2, key_dim=128, value_dim=48, taps=4)
+    channels, inner = 2 * 2 * 128 + 4 * 48, 4 * 48
+    generator = torch.Generator(DEVICE).manual_seed(portion)
+    normal = lambda *shape: torch.randn(shape, generator=generator, device=DEVICE)
+    constants = dict(conv=0.5 * normal(channels, 4), a_log=normal(4) - 2, dt_bias=normal(4),
+                     norm_weight=1 + 0.2 * normal(48), eps=1e-5, unit_eps=1e-6, write=True, **sizes)
+    rows = normal(sum(beside) + portion, channels + inner + 8)
+    size = GatedDeltaRule.state_size(sizes)
+    kept = normal(len(beside) + 1, size)
+    results = []
+    for portions in ([portion], list(beside) + [portion]):
+        n = len(portions)
+        state = kept[-n:].clone()
+        ctx = context(portions, [9] * n)
+        ctx.leading_single = lead if n > 1 and portion > 1 else 0
+        # (one token by itself runs in the kernel of single tokens: here it is a portion all the same)
+        ctx.max_portion = max(ctx.max_portion, 2)
+        view = StateView(state, torch.arange(n, dtype=torch.int32, device=DEVICE), FixedState((size,), "float32"))
+        out = ops.gated_delta_rule(rows[-sum(portions):].contiguous(), ctx=ctx, view=view, **constants)
+        results.append((out[-portion:].clone(), state[-1].clone()))
+    ops.check_errors()
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
