@@ -202,8 +202,10 @@ attention_f32_kernel(const float* q, const float* kv, const int* block_table, in
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const int j = tx + 16 * c;
-                    const bool live = j < seen[i] && row_of[j] >= 0 && unit_max[i] != -INFINITY;
-                    const float weight = live ? expf(score[i][c] - unit_max[i]) : 0.f;
+                    // (a maximum of nothing but NaN is -inf too: the weights stay NaN)
+                    const bool live = j < seen[i] && row_of[j] >= 0;
+                    const float weight =
+                        live ? expf(score[i][c] - (unit_max[i] == -INFINITY ? 0.f : unit_max[i])) : 0.f;
                     weights[(ty * RPT + i) * (UNIT + 1) + j] = weight;
                     total += weight;
                 }
@@ -257,7 +259,7 @@ attention_f32_kernel(const float* q, const float* kv, const int* block_table, in
                         for (int d = 0; d < DIMS; ++d) to[tx * DIMS + d] = mixed[i][d];
                         if (tx == 0) { to[D] = unit_max[i]; to[D + 1] = unit_sum[i]; }
                     }
-                } else if (unit_max[i] != -INFINITY) {
+                } else if (seen[i] > 0 && fmaxf(max_so_far[i], unit_max[i]) != -INFINITY) {
                     const Joint join(max_so_far[i], unit_max[i]);
                     max_so_far[i] = join.max;
                     sum[i] = join(sum[i], unit_sum[i]);
@@ -296,8 +298,8 @@ __global__ void __launch_bounds__(D) attention_f32_merge_kernel(const float* par
 #pragma unroll 4
     for (int unit = 0; unit < count; ++unit, from += D + 4) {
         const float value = __ldcg(from + d), unit_max = __ldcg(from + D), unit_sum = __ldcg(from + D + 1);
-        if (unit_max == -INFINITY) continue;
         const Joint join(max_so_far, unit_max);
+        if (join.max == -INFINITY) continue;
         max_so_far = join.max;
         sum = join(sum, unit_sum);
         acc = join(acc, value);

@@ -130,3 +130,31 @@ def test_positions_behind_the_table(ops, portions):
                 ops.check_errors()
     finally:
         ops._sm_count = count
+
+
+@pytest.mark.parametrize("portions,histories,spoilt", [([1], [128], range(128, 129)), ([1, 1], [200, 70], range(128, 192)),
+                                                       ([40], [100], range(128, 129)), ([70], [128], range(64, 128))])
+def test_scores_that_are_nan(ops, portions, histories, spoilt):
+    """Keys that are NaN, all of a unit of 64 or all that a query sees of it: every query that sees one is NaN,
+    the others keep their bits."""
+    page, heads, kv_heads, dim = 16, 4, 2, 32
+    ctx, table, pages = make_batch(portions, histories, page, DEVICE)
+    generator = torch.Generator(DEVICE).manual_seed(7)
+    kv = torch.randn(2, pages, kv_heads, page, dim, generator=generator, device=DEVICE)
+    q = torch.randn(ctx.tokens, heads, dim, generator=generator, device=DEVICE)
+    view = PagedView(kv, table, page, PagedKeyValues(kv_heads, dim, None))
+    attend = lambda: ops.paged_attention(q, heads=heads, kv_heads=kv_heads, head_dim=dim, scale=0.2, window=None,
+                                         ctx=ctx, view=view)
+    count = ops._sm_count
+    try:
+        for ops._sm_count in (0, 1 << 30):
+            view.kv = kv.clone()
+            want = attend()
+            for at in spoilt:
+                view.kv[0, int(table[0, at // page]), :, at % page] = float("nan")
+            got = attend()
+            sees = (ctx.token_request == 0) & (ctx.positions >= spoilt[0])
+            assert torch.isnan(got[sees]).all() and torch.equal(got[~sees], want[~sees])
+    finally:
+        ops._sm_count = count
+    ops.check_errors()
