@@ -2,6 +2,7 @@
 than the engine's tiny models: head sizes in steps of 16, odd head counts and groups, widths
 and vocabularies that are no power of two."""
 
+import ctypes
 import math
 
 import pytest
@@ -95,6 +96,19 @@ def test_gather_swiglu_bias(ops, plain, dtype):
     gate_up = torch.randn(29, 2 * 77).to(dtype)
     torch.testing.assert_close(ops.swiglu(gate_up.to(DEVICE)).cpu().float(),
                                plain.swiglu(gate_up).float(), **tolerance(dtype))
+
+
+@pytest.mark.parametrize("width", [8, 24, 31, 2056])
+def test_bias_of_some_columns(ops, width):
+    """A bias that is zero in some columns: every value is value + bias, rounded once, signs of zeros too."""
+    x = torch.randn(37, width, device=DEVICE).bfloat16()
+    x[::3] = -0.0
+    bias = torch.randn(width, device=DEVICE)
+    bias[width // 3:] = 0.0
+    got, want = x.clone(), (x.float() + bias).bfloat16()
+    ops._call("mlxone_add_bias", *(ctypes.c_void_p(t.data_ptr()) for t in (got, bias)), ctypes.c_int(37),
+              ctypes.c_int(width), ctypes.c_int(1))
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
 
 
 @pytest.mark.parametrize("m,n,k", [(1, 5, 7), (37, 333, 130), (64, 96, 288), (130, 1000, 96)])
