@@ -117,6 +117,9 @@ class CudaOps:
         self.skinny_fused_max_rows = 16
         # latent attention of few tokens: the key up-projection with the queries' rotation in one kernel
         self.fused_latent = True
+        # 32-bit attention with the units of keys side by side: scratch values of a launch (64 MB).
+        # A kept graph of a step holds its own.
+        self.split_scratch = 1 << 24
         # The delta rule with keys of 128 values: portions from this length on are worked on in chunks of
         # 32 tokens, shorter ones four tokens at a time. Microseconds a layer by chunks / by fours, 16
         # heads of 128 x 128: one portion of 32 / 48 / 64 / 333 tokens 25 / 20, 27 / 24, 28 / 29, 53 /
@@ -1732,7 +1735,9 @@ class CudaOps:
     def _attention_f32(self, q, out, heads, kv_heads, head_dim, scale, ctx, view):
         """The 32-bit engine's attention over every earlier key: single tokens and portions each
         by a launch of their own, one block per unit of 64 keys where whole rows would be too few
-        blocks for two on every SM (one token of a request at position 140: 8 blocks or 24)."""
+        blocks for two on every SM (one token of a request at position 140: 8 blocks or 24). The
+        units' sums lie in scratch of up to ``split_scratch`` values (more only where a tile of
+        tokens by itself needs more); tokens that need more go one part after the other."""
         tokens, width = q.shape[0], view.block_table.shape[1]
         if ctx.max_portion == 1 and tokens == ctx.requests:
             singles = tokens
@@ -1745,20 +1750,25 @@ class CudaOps:
         for first, end, single in ((0, singles, 1), (singles, tokens, 0)):
             if first == end:
                 continue
-            tiles = end - first if single else -(-(end - first) // (32 // group))
-            values = (end - first) * heads * units * (head_dim + 4)
-            partial = None
-            if 1 < units <= 65535 and tiles * kv_heads < 2 * self._sm_count and values <= 1 << 26:
-                partial = torch.empty(values, dtype=torch.float32, device=self.device)
-            self._call("mlxone_attention_f32", _c_void_p(_ptr(q)), _c_void_p(_ptr(view.kv)),
-                       _c_void_p(_ptr(view.block_table)), _c_int(width), _c_int(view.page_size),
-                       _c_int(view.kv.shape[1]), _c_void_p(_ptr(ctx.positions)),
-                       _c_void_p(_ptr(ctx.token_request)), _c_void_p(_ptr(out)),
-                       _c_void_p(_ptr(partial)), _c_int(first), _c_int(end), _c_int(single),
-                       _c_int(0 if partial is None else units), _c_int(heads), _c_int(kv_heads),
-                       _c_int(head_dim), _c_float(scale), _c_void_p(_ptr(self.error_flag)))
-            if partial is not None:
-                self.launches += 1          # the merge kernel
+            tile = 1 if single else 32 // group
+            values = heads * units * (head_dim + 4)          # of scratch, a token
+            cut, partial = end - first, None
+            if (1 < units <= 65535 and -(-cut // tile) * kv_heads < 2 * self._sm_count
+                    and cut * values <= 1 << 26):
+                # (whole tiles of tokens at a time, one launch after the other in one scratch)
+                cut = min(cut, max(self.split_scratch // values // tile, 1) * tile)
+                partial = torch.empty(cut * values, dtype=torch.float32, device=self.device)
+            for at in range(first, end, cut):
+                self._call("mlxone_attention_f32", _c_void_p(_ptr(q)), _c_void_p(_ptr(view.kv)),
+                           _c_void_p(_ptr(view.block_table)), _c_int(width), _c_int(view.page_size),
+                           _c_int(view.kv.shape[1]), _c_void_p(_ptr(ctx.positions)),
+                           _c_void_p(_ptr(ctx.token_request)), _c_void_p(_ptr(out)),
+                           _c_void_p(_ptr(partial)), _c_int(at), _c_int(min(at + cut, end)),
+                           _c_int(single), _c_int(0 if partial is None else units), _c_int(heads),
+                           _c_int(kv_heads), _c_int(head_dim), _c_float(scale),
+                           _c_void_p(_ptr(self.error_flag)))
+                if partial is not None:
+                    self.launches += 1          # the merge kernel
 
     def _shaped_attention(self, q, heads, kv_heads, head_dim, scale, ctx, view, cap, slopes, least_slope):
         """paged_attention with capped or distance-biased scores, on the same kernels built with the

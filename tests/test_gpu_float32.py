@@ -158,3 +158,32 @@ def test_scores_that_are_nan(ops, portions, histories, spoilt):
     finally:
         ops._sm_count = count
     ops.check_errors()
+
+
+def test_scratch_of_units_side_by_side(ops):
+    """Tokens whose units would not fit the scratch together go one part after the other: the same bits,
+    and no more memory than stated, down to one tile of tokens at a time."""
+    heads, kv_heads, dim, page = 16, 4, 64, 16
+    ctx, table, pages = make_batch([1, 1, 1, 150], [3000, 5, 64, 2900], page, DEVICE)
+    ctx.leading_single = 3
+    generator = torch.Generator(DEVICE).manual_seed(2)
+    kv = torch.randn(2, pages, kv_heads, page, dim, generator=generator, device=DEVICE)
+    q = torch.randn(ctx.tokens, heads, dim, generator=generator, device=DEVICE)
+    view = PagedView(kv, table, page, PagedKeyValues(kv_heads, dim, None))
+    kept, results = ops.split_scratch, []
+    tile = 32 // (heads // kv_heads) * heads * -(-table.shape[1] * page // 64) * (dim + 4)
+    try:
+        for ops.split_scratch in (kept, 3 * tile + 5, 1):
+            torch.cuda.reset_peak_memory_stats()
+            base, before = torch.cuda.memory_allocated(), ops.launches
+            results.append(ops.paged_attention(q, heads=heads, kv_heads=kv_heads, head_dim=dim, scale=0.1,
+                                               window=None, ctx=ctx, view=view))
+            peak = torch.cuda.max_memory_allocated() - base - 4 * q.numel()
+            # (the allocator hands out blocks whole that are up to 1 MB larger)
+            assert peak <= 4 * max(tile, ops.split_scratch) + (1 << 20)
+            # singles and portion, each with its merge; tiles of 8 tokens, three or one at a time
+            assert ops.launches - before == {kept: 4, 1: 2 * 3 + 2 * 19}.get(ops.split_scratch, 2 + 2 * 7)
+    finally:
+        ops.split_scratch = kept
+    assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
+    ops.check_errors()
