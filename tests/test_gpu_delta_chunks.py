@@ -130,3 +130,46 @@ def test_a_portion_does_not_depend_on_its_neighbours(ops, portion, chunk_from, b
         results.append((out[-portion:].clone(), state[-1].clone()))
     ops.check_errors()
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("offset", [0, 2])
+def test_values_of_128(ops, dtype, offset):
+    """Eight tiles of columns in the walk, the largest block of the single-token kernel, and the output's norm
+    four values a lane, or one where the rows do not allow it (``offset``): portions, single tokens, portions."""
+    from mlx_one_b200.parts import FixedState, StateView
+    from mlx_one_b200.parts.mixers import GatedDeltaRule
+
+    H, G, D, V, taps = 4, 2, 128, 128, 4
+    sizes = dict(heads=H, kv_heads=G, key_dim=D, value_dim=V, taps=taps)
+    channels, inner = 2 * G * D + H * V, H * V
+    width = channels + inner + 2 * H
+    generator = torch.Generator().manual_seed(11)
+    steps = [(70, 33), (1, 1), (1, 1), (1, 1), (2, 1), (65, 64), (1, 1)]
+    lengths = [sum(step[r] for step in steps) for r in (0, 1)]
+    projected = [(1.5 * torch.randn(n, width, generator=generator)).to(dtype) for n in lengths]
+    conv = 0.5 * torch.randn(channels, taps, generator=generator)
+    a_log, dt_bias = torch.randn(H, generator=generator) - 2, torch.randn(H, generator=generator)
+    norm_weight = 1 + 0.2 * torch.randn(V, generator=generator)
+    size = GatedDeltaRule.state_size(sizes)
+    view = StateView(torch.zeros(2, size, device=DEVICE), torch.tensor([1, 0], dtype=torch.int32, device=DEVICE),
+                     FixedState((size,), "float32"))
+    constants = dict(conv=conv.to(DEVICE), a_log=a_log.to(DEVICE), dt_bias=dt_bias.to(DEVICE),
+                     norm_weight=norm_weight.to(DEVICE), eps=1e-5, unit_eps=1e-6, view=view, write=True, **sizes)
+    got, fed = [[], []], [0, 0]
+    for step in steps:
+        wide = torch.zeros(sum(step), width + 8, dtype=dtype, device=DEVICE)
+        rows = wide[:, offset:offset + width]
+        rows.copy_(torch.cat([projected[r][fed[r]:fed[r] + step[r]] for r in (0, 1)]))
+        ctx = context(list(step), list(fed))
+        ctx.leading_single = 2 if max(step) == 1 else 0
+        out = ops.gated_delta_rule(rows, ctx=ctx, **constants)
+        got[0].append(out[:step[0]].cpu())
+        got[1].append(out[step[0]:].cpu())
+        fed = [fed[r] + step[r] for r in (0, 1)]
+    ops.check_errors()
+    for r in (0, 1):
+        want = delta_pieces(projected[r].double(), conv.double(), a_log.double(), dt_bias.double(),
+                            norm_weight.double(), 1e-5, sizes)
+        # (the bounds of the test above)
+        assert (torch.cat(got[r]).double() - want).abs().max() < bound(dtype, 5e-5, 0.1), f"request {r}"

@@ -40,3 +40,49 @@ def test_same_logits_with_dependent_launches(tmp_path, name):
     finally:
         ops.set_dependent_launches(True)
     assert torch.equal(results[0], results[1])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("name", ["B", "D", "G1", "G2", "G3", "G5"])
+def test_same_logits_in_32_bit_and_with_the_delta_rule(tmp_path, name, dtype):
+    """The 32-bit engine's kernels and the delta rule's: portions, single tokens beside a portion, single
+    tokens step by step and in a loop without the host."""
+    import galarax_models
+    from mlx_one_b200.cache import CacheManager
+    from mlx_one_b200.engine.loading import load_model
+    from mlx_one_b200.engine.runner import Runner, StepEntry
+
+    if name in CONFIGS:
+        vocab, folder = CONFIGS[name][0]["vocab_size"], make_model_dir(name, tmp_path, dtype=dtype)
+    else:
+        vocab, folder = galarax_models.CONFIGS[name][0]["vocab"], galarax_models.make_model_dir(name, tmp_path)
+    loaded = load_model(folder, dtype, "cuda:0")
+    ops = loaded.model.ops
+    requests = prompts(vocab, (90, 15, 77), seed=9)
+    late = prompts(vocab, (70,), seed=10)[0]
+    results = []
+    try:
+        for enabled in (False, True):
+            ops.set_dependent_launches(enabled)
+            cache = CacheManager(loaded.model.cache_needs, page_size=8, capacity_tokens=1024, max_requests=4,
+                                 dtype=dtype, device="cuda:0")
+            runner = Runner(loaded.model, cache)
+            for i in range(4):
+                cache.open(i)
+            collected = []
+
+            def step(entries):
+                collected.append(runner.step(entries).float().cpu().clone())
+
+            step([StepEntry(i, tokens[:-8], (0,)) for i, tokens in enumerate(requests)])
+            for at in range(-8, 0):
+                step([StepEntry(i, [tokens[at]], (0,)) for i, tokens in enumerate(requests)] +
+                     ([StepEntry(3, late, (69,))] if at == -4 else []))
+            chosen = runner.decode_steps([StepEntry(i, [5], (0,)) for i in range(4)], 40)
+            collected.append(chosen.float().cpu())
+            step([StepEntry(i, [6], (0,)) for i in range(4)])
+            ops.check_errors()
+            results.append(collected)
+    finally:
+        ops.set_dependent_launches(True)
+    assert all(torch.equal(a, b) for a, b in zip(*results))

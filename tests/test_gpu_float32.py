@@ -34,6 +34,25 @@ def test_products_of_any_number_of_rows(ops, n, k):
             assert torch.equal(got[0], first), (m, a.stride())
 
 
+@pytest.mark.parametrize("n,k", [(2500, 4608), (2501, 2056), (5000, 1032), (9500, 520)])
+def test_products_walk_groups_and_sections(ops, n, k):
+    """Weights streamed by warps that take several groups of rows and several sections of K each, with the
+    rows of the input brought in one or several parts: every row has the bits that the tiles give it."""
+    generator = torch.Generator(DEVICE).manual_seed(n + k)
+    normal = lambda *shape: torch.randn(shape, generator=generator, device=DEVICE)
+    a, w, bias = normal(130, k), normal(n, k), normal(n)
+    tiles = ops.linear(a, w, bias)
+    want = a.double() @ w.double().T + bias.double()
+    bound = (32 + k / 256 + 10) * 2.0 ** -24 * (a.abs().double() @ w.abs().double().T + bias.abs().double())
+    assert ((tiles.double() - want).abs() <= bound).all()
+    for m in (1, 2, 3, 4, 7, 8, 9, 17, 32, 33, 64):
+        assert torch.equal(ops.linear(a[:m], w, bias), tiles[:m]), m
+    # weights that are aligned to 16 bytes only: tiles at every number of rows
+    shifted = torch.empty(n * k + 4, device=DEVICE)[4:].view(n, k).copy_(w)
+    for m in (1, 8, 17):
+        assert torch.equal(ops.linear(a[:m], shifted, bias), tiles[:m]), m
+
+
 @pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [
     (16, 8, 64, 16), (24, 8, 64, 16), (4, 4, 32, 4), (12, 1, 128, 32), (32, 1, 64, 64)])
 @pytest.mark.parametrize("portions,histories", [
