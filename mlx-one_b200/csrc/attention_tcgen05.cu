@@ -39,6 +39,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "float_pairs.cuh"
 #include "score_shape.cuh"
 
 namespace {
@@ -195,33 +196,9 @@ __device__ __forceinline__ float fast_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// Two 32-bit floats in one instruction (fma.rn.f32x2, add.rn.f32x2) and a maximum of three: the
-// softmax warps issue about one instruction less per score for each of them, and their issue
-// slots are what a tile's softmax costs beside its exponentials.
-__device__ __forceinline__ unsigned long long pair_of(float lo, float hi) {
-    unsigned long long v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ void unpair(unsigned long long v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b,
-                                                       unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ unsigned long long mul_pair(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long add_pair(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
+// Pairs of floats (float_pairs.cuh) and a maximum of three: the softmax warps issue about one instruction
+// less per score for each of them, and their issue slots are what a tile's softmax costs beside its
+// exponentials.
 __device__ __forceinline__ float max_of_three(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));

@@ -32,6 +32,7 @@
 // the products of the decay's and the gate's second matrices (their rows for this head are asked
 // for before the wait for the projection).
 #include "delta_common.cuh"
+#include "float_pairs.cuh"
 
 namespace {
 
@@ -45,27 +46,6 @@ constexpr int SOLVE = 2 * GROUP * GROUP;    // M, then Q, both [GROUP][GROUP]
 constexpr int STEP_LANES = 4;        // single-token kernel: lanes that share a column of S
 constexpr int STEP_MAX_COLUMNS = 128;
 constexpr int STEP_ROWS = 16;        // rows of the second matrices that a warp holds in registers
-
-// Two 32-bit numbers in one register pair.
-using Pair = unsigned long long;
-__device__ __forceinline__ Pair pair_of(float lo, float hi) {
-    Pair p;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
-    return p;
-}
-__device__ __forceinline__ void halves(Pair p, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
-}
-__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
-    Pair d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
-    Pair d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 
 __device__ __forceinline__ float sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
 
@@ -388,7 +368,7 @@ channel_scan_kernel(const float* __restrict__ kc, const float* __restrict__ qc,
     const int lane = threadIdx.x & (LANES - 1), team = threadIdx.x / LANES;
     const int column0 = blockIdx.x * COLUMNS + team * COLS;
     float* matrix = slot + (size_t)h * D * V;
-    Pair S[COLS][PER / 2];                            // rows 2 e and 2 e + 1 of this lane's
+    FloatPair S[COLS][PER / 2];                            // rows 2 e and 2 e + 1 of this lane's
     auto stored = [&](int c, int e) {
         const int row = lane * PER + e;
         return column0 + c < V && row < D ? matrix[(size_t)row * V + column0 + c] : 0.f;
@@ -458,26 +438,26 @@ channel_scan_kernel(const float* __restrict__ kc, const float* __restrict__ qc,
             float sum[2 * PAIRS];
 #pragma unroll
             for (int j = 0; j < GROUP; ++j) {
-                Pair a[COLS], b[COLS];
+                FloatPair a[COLS], b[COLS];
 #pragma unroll
                 for (int e = 0; e < PER; e += 4) {
                     const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kcs + (t0 + j) * ROWS + lane * PER + e);
                     const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qcs + (t0 + j) * ROWS + lane * PER + e);
 #pragma unroll
                     for (int c = 0; c < COLS; ++c) {
-                        a[c] = e == 0 ? pair_mul(S[c][0], k4.x) : pair_fma(S[c][e / 2], k4.x, a[c]);
-                        b[c] = e == 0 ? pair_mul(S[c][0], q4.x) : pair_fma(S[c][e / 2], q4.x, b[c]);
-                        a[c] = pair_fma(S[c][e / 2 + 1], k4.y, a[c]);
-                        b[c] = pair_fma(S[c][e / 2 + 1], q4.y, b[c]);
+                        a[c] = e == 0 ? mul_pair(S[c][0], k4.x) : fma_pair(S[c][e / 2], k4.x, a[c]);
+                        b[c] = e == 0 ? mul_pair(S[c][0], q4.x) : fma_pair(S[c][e / 2], q4.x, b[c]);
+                        a[c] = fma_pair(S[c][e / 2 + 1], k4.y, a[c]);
+                        b[c] = fma_pair(S[c][e / 2 + 1], q4.y, b[c]);
                     }
                 }
 #pragma unroll
                 for (int c = 0; c < COLS; ++c) {
                     const int pair = c * GROUP + j;
                     float lo, hi;
-                    halves(a[c], lo, hi);
+                    unpair(a[c], lo, hi);
                     sum[SPLIT ? pair : 2 * pair] = lo + hi;
-                    halves(b[c], lo, hi);
+                    unpair(b[c], lo, hi);
                     sum[SPLIT ? PAIRS + pair : 2 * pair + 1] = lo + hi;
                 }
             }
@@ -525,13 +505,13 @@ channel_scan_kernel(const float* __restrict__ kc, const float* __restrict__ qc,
                 const ulonglong2 c4 = *reinterpret_cast<const ulonglong2*>(cums + (t0 / GROUP) * ROWS + lane * PER + e);
 #pragma unroll
                 for (int c = 0; c < COLS; ++c) {
-                    S[c][e / 2] = pair_mul(S[c][e / 2], c4.x);
-                    S[c][e / 2 + 1] = pair_mul(S[c][e / 2 + 1], c4.y);
+                    S[c][e / 2] = mul_pair(S[c][e / 2], c4.x);
+                    S[c][e / 2 + 1] = mul_pair(S[c][e / 2 + 1], c4.y);
                 }
             }
 #pragma unroll
             for (int j = 0; j < GROUP; j += 4) {
-                Pair u[COLS][4];
+                FloatPair u[COLS][4];
 #pragma unroll
                 for (int c = 0; c < COLS; ++c) {
                     const float4 w = *reinterpret_cast<const float4*>(own + PAIRS + c * GROUP + j);
@@ -545,8 +525,8 @@ channel_scan_kernel(const float* __restrict__ kc, const float* __restrict__ qc,
                         const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kss + (t0 + j + step) * ROWS + lane * PER + e);
 #pragma unroll
                         for (int c = 0; c < COLS; ++c) {
-                            S[c][e / 2] = pair_fma(k4.x, u[c][step], S[c][e / 2]);
-                            S[c][e / 2 + 1] = pair_fma(k4.y, u[c][step], S[c][e / 2 + 1]);
+                            S[c][e / 2] = fma_pair(k4.x, u[c][step], S[c][e / 2]);
+                            S[c][e / 2 + 1] = fma_pair(k4.y, u[c][step], S[c][e / 2 + 1]);
                         }
                     }
                 }
@@ -563,7 +543,7 @@ channel_scan_kernel(const float* __restrict__ kc, const float* __restrict__ qc,
             for (int c = 0; c < COLS; ++c) {
                 const int row = lane * PER + e;
                 float lo, hi;
-                halves(S[c][e / 2], lo, hi);
+                unpair(S[c][e / 2], lo, hi);
                 if (column0 + c < V && row < D) matrix[(size_t)row * V + column0 + c] = lo;
                 if (column0 + c < V && row + 1 < D) matrix[(size_t)(row + 1) * V + column0 + c] = hi;
             }

@@ -15,6 +15,7 @@
 #pragma once
 
 #include "delta_common.cuh"
+#include "float_pairs.cuh"
 
 namespace {
 
@@ -40,29 +41,10 @@ __device__ __forceinline__ void copy_or_zero_16(float* dst, const float* src, bo
                  : "memory");
 }
 
-typedef unsigned long long FloatPair;
-__device__ __forceinline__ FloatPair pair_of(float x) {
-    FloatPair p;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(p) : "f"(x));
-    return p;
-}
-__device__ __forceinline__ FloatPair pair_of(float x, float y) {
-    FloatPair p;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(x), "f"(y));
-    return p;
-}
-__device__ __forceinline__ FloatPair mul_pair(FloatPair x, FloatPair y) {
-    FloatPair p;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(x), "l"(y));
-    return p;
-}
-__device__ __forceinline__ void fma_pair(FloatPair& acc, FloatPair x, FloatPair y) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y));
-}
 __device__ __forceinline__ float4 quad_of(FloatPair a, FloatPair b) {
     float4 v;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(a));
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.z), "=f"(v.w) : "l"(b));
+    unpair(a, v.x, v.y);
+    unpair(b, v.z, v.w);
     return v;
 }
 
@@ -248,8 +230,8 @@ __device__ __forceinline__ void chunk_product(const float* x, int pitch, const f
             for (int e = 0; e < 4; ++e) {
                 if (LOWER && column + step * 4 + e > (rg + 8 * i) % DC) continue;
                 const FloatPair f = pair_of(values[e]);
-                fma_pair(acc[i][0], f, b[e].x);
-                fma_pair(acc[i][1], f, b[e].y);
+                accumulate_pair(acc[i][0], f, b[e].x);
+                accumulate_pair(acc[i][1], f, b[e].y);
             }
         }
     }
@@ -399,8 +381,8 @@ delta_walk_kernel(const float* q_in, const float* k_in, const float* v_in, const
                 const FloatPair ks[4] = {pair_of(k.x), pair_of(k.y), pair_of(k.z), pair_of(k.w)};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    fma_pair(S[i][0], ks[i], u.x);
-                    fma_pair(S[i][1], ks[i], u.y);
+                    accumulate_pair(S[i][0], ks[i], u.x);
+                    accumulate_pair(S[i][1], ks[i], u.y);
                 }
             }
 #pragma unroll

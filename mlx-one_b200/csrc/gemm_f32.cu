@@ -14,6 +14,7 @@
 // rows, its lanes need nothing from one another inside a section, and a tile that walks a strand
 // still fetches whole 32-byte sectors.
 #include "common.cuh"
+#include "float_pairs.cuh"
 
 #include <algorithm>
 
@@ -190,25 +191,6 @@ gemm_f32_skinny_kernel(const float* a, int lda, const float* __restrict__ w, int
 // tile keeps an SM busy where there are few tiles), and the sections' sums meet in shared memory, in
 // order. Within a group: stages of BK values of K (16: two pieces of a strand, 32: all four), K
 // outermost in shared memory, double-buffered, the next stage's values under way in registers.
-typedef unsigned long long Pair;
-
-__device__ __forceinline__ Pair both(float x) {
-    Pair p;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(p) : "f"(x));
-    return p;
-}
-__device__ __forceinline__ void fma_pair(Pair& acc, Pair x, Pair y) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y));
-}
-__device__ __forceinline__ void add_pair(Pair& acc, Pair x) {
-    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(x));
-}
-__device__ __forceinline__ float2 halves(Pair p) {
-    float2 v;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
-    return v;
-}
-
 template <int BM, int BN, int TM, int TN, int G, int BK, bool VEC>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN) * G)
 gemm_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw,
@@ -318,7 +300,7 @@ gemm_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ 
     }
     for (int round = 0; round < rounds; ++round) {
         const int section = round * G + group;
-        Pair sum[TM][TN / 2];
+        FloatPair sum[TM][TN / 2];
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -326,7 +308,7 @@ gemm_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ 
         if (section < sections) {
             const int deep = stages_of(section);
             for (int strand = 0; strand < STRANDS; ++strand) {
-                Pair acc[TM][TN / 2];
+                FloatPair acc[TM][TN / 2];
 #pragma unroll
                 for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -341,11 +323,11 @@ gemm_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ 
                     const float* ws = stages + buffer * STAGE + BK * (BM + 4) + tx * 4;
 #pragma unroll
                     for (int kk = 0; kk < BK; ++kk) {
-                        Pair x[TM], y[TN / 2];
+                        FloatPair x[TM], y[TN / 2];
 #pragma unroll
                         for (int i = 0; i < TM; i += 4) {
                             const float4 v = *reinterpret_cast<const float4*>(as + kk * (BM + 4) + i * (BM / TM));
-                            x[i] = both(v.x); x[i + 1] = both(v.y); x[i + 2] = both(v.z); x[i + 3] = both(v.w);
+                            x[i] = pair_of(v.x); x[i + 1] = pair_of(v.y); x[i + 2] = pair_of(v.z); x[i + 3] = pair_of(v.w);
                         }
 #pragma unroll
                         for (int j = 0; j < TN; j += 4) {
@@ -356,7 +338,7 @@ gemm_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ 
 #pragma unroll
                         for (int i = 0; i < TM; ++i)
 #pragma unroll
-                            for (int j = 0; j < TN / 2; ++j) fma_pair(acc[i][j], x[i], y[j]);
+                            for (int j = 0; j < TN / 2; ++j) accumulate_pair(acc[i][j], x[i], y[j]);
                     }
                     buffer ^= 1;
                     if (more) store(buffer);
@@ -365,14 +347,15 @@ gemm_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ 
 #pragma unroll
                 for (int i = 0; i < TM; ++i)
 #pragma unroll
-                    for (int j = 0; j < TN / 2; ++j) add_pair(sum[i][j], acc[i][j]);
+                    for (int j = 0; j < TN / 2; ++j) accumulate_pair(sum[i][j], acc[i][j]);
             }
         }
         if (G == 1) {
 #pragma unroll
             for (int i = 0; i < PAIRS; ++i) {
                 float2 total = totals[i * THREADS + tid];
-                const float2 here = halves(sum[i / (TN / 2)][i % (TN / 2)]);
+                float2 here;
+                unpair(sum[i / (TN / 2)][i % (TN / 2)], here.x, here.y);
                 total.x += here.x;
                 total.y += here.y;
                 totals[i * THREADS + tid] = total;
@@ -380,8 +363,11 @@ gemm_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ 
         } else {
             if (round > 0) __syncthreads();        // the last round's parts have been read
 #pragma unroll
-            for (int i = 0; i < PAIRS; ++i)
-                parts[(group * PAIRS + i) * THREADS + tid] = halves(sum[i / (TN / 2)][i % (TN / 2)]);
+            for (int i = 0; i < PAIRS; ++i) {
+                float2 here;
+                unpair(sum[i / (TN / 2)][i % (TN / 2)], here.x, here.y);
+                parts[(group * PAIRS + i) * THREADS + tid] = here;
+            }
             __syncthreads();
             const int here = min(G, sections - round * G);
             for (int i = group; i < PAIRS; i += G) {
