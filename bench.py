@@ -2365,6 +2365,28 @@ def kernel_case(name: str, batch: int, context: int) -> int:
         w = weights(2 * width, hidden, 2)
         run = lambda i: ops.linear_swiglu(a, w[i % 2])
         work = f"{2 * PREFILL_TOKENS * 2 * width * hidden / 1e9:.1f} GFLOP"
+    elif name == "tcgen05_swiglu_narrow":
+        # the same product at a size that takes tiles of 96 + 96 rows of the weights
+        a = torch.randn(424, 1536, device=device).bfloat16()
+        w = weights(2 * 6912, 1536, 4)
+        run = lambda i: ops.linear_swiglu(a, w[i % 4])
+        work = f"{2 * 424 * 2 * 6912 * 1536 / 1e9:.1f} GFLOP"
+    elif name == "product_f32":
+        # the 32-bit product: weights streamed for up to 32 rows, tiles beyond
+        a = torch.randn(batch, hidden, device=device)
+        w = [x.float() for x in weights(2 * width, hidden, 2)]
+        run = lambda i: ops.linear(a, w[i % 2])
+        work = (f"{batch} rows, {2 * width * hidden * 4 / 1e6:.1f} MB of weights, "
+                f"{2 * batch * 2 * width * hidden / 1e9:.1f} GFLOP")
+    elif name in ("attention_f32_prefill", "attention_f32_decode"):
+        portions = [300] * batch if name == "attention_f32_prefill" else [1] * batch
+        ctx, view = batch_context(portions, [0 if portions[0] > 1 else context - 1] * batch)
+        ctx.leading_single = batch if portions[0] == 1 else 0
+        view.kv = view.kv.float()
+        q = torch.randn(ctx.tokens, heads, head_dim, device=device)
+        run = lambda i: ops.paged_attention(q, heads=heads, kv_heads=kv_heads, head_dim=head_dim,
+                                            scale=head_dim ** -0.5, window=None, ctx=ctx, view=view)
+        work = f"{ctx.tokens} tokens of {batch} requests, {heads} heads over {kv_heads} of {head_dim}"
     elif name == "swapped_swiglu":
         # the 33-to-128-row product with swapped operands (an option, off by default) on w13
         rows = max(batch, 33)
@@ -2396,9 +2418,10 @@ def kernel_case(name: str, batch: int, context: int) -> int:
         steps = torch.zeros(batch, dtype=torch.int32, device=device)
         run = lambda i: ops.sample(logits[i % 4], temperature, top_k, top_p, seed, steps)
         work = f"{batch} rows of {vocab} logits, temperature 0.8, top-k 40, top-p 0.9"
-    elif name in ("delta_prefill", "delta_decode"):
+    elif name in ("delta_prefill", "delta_short", "delta_decode"):
         # the gated delta rule alone: 16 heads of 128 x 128, a prompt of 2048 tokens (prepare,
-        # scan, finish) or `batch` single tokens (one kernel)
+        # chunks, walk, finish), `batch` portions of 48 tokens (prepare, scan, finish) or `batch`
+        # single tokens (one kernel)
         from mlx_one_b200.parts import FixedState, StateView
         from mlx_one_b200.parts.mixers import GatedDeltaRule
 
@@ -2406,8 +2429,9 @@ def kernel_case(name: str, batch: int, context: int) -> int:
         slot = GatedDeltaRule.state_size(sizes)
         channels = 2 * 8 * 128 + 16 * 128
         wide = channels + 16 * 128 + 2 * 16
-        portions = [PREFILL_TOKENS] if name == "delta_prefill" else [1] * batch
-        ctx, _ = batch_context(portions, [0 if name == "delta_prefill" else context] * len(portions))
+        portions = {"delta_prefill": [PREFILL_TOKENS], "delta_short": [48] * batch,
+                    "delta_decode": [1] * batch}[name]
+        ctx, _ = batch_context(portions, [context if name == "delta_decode" else 0] * len(portions))
         state = torch.zeros(4 * len(portions), slot, device=device)
         views = [StateView(state, torch.arange(c * len(portions), (c + 1) * len(portions),
                                                dtype=torch.int32, device=device),
@@ -2670,7 +2694,9 @@ def main() -> int:
     parser.add_argument("--kernel", default=None,
                         help="run one kernel alone instead of the benchmark: skinny_swiglu, "
                              "skinny_in_proj, skinny_down, decode_attention, prefill_attention, tcgen05_swiglu, "
-                             "swapped_swiglu, mixed_attention, sampling, delta_prefill, delta_decode, lightning_prefill, "
+                             "tcgen05_swiglu_narrow, product_f32, attention_f32_prefill, attention_f32_decode, "
+                             "swapped_swiglu, mixed_attention, sampling, delta_prefill, delta_short, delta_decode, "
+                             "lightning_prefill, "
                              "lightning_decode, experts_sorted, latent_prefill, latent_decode, state_space_prefill, "
                              "state_space_decode, channel_conv_prefill, channel_delta_prefill, "
                              "channel_delta_decode, recurrence_prefill, recurrence_decode, "

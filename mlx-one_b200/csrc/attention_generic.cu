@@ -11,7 +11,8 @@
 // first, the blocks between them and the window's first are skipped. With SHAPED a score passes a cap
 // and a distance bias ahead of the softmax (score_shape.cuh).
 //
-// This kernel serves the 32-bit engine and every shape that the faster kernels refuse.
+// This kernel serves every call that the faster kernels refuse: in 32-bit windows, sinks, shaped scores and
+// head sizes other than 32, 64 and 128.
 #include "common.cuh"
 #include "score_shape.cuh"
 

@@ -25,8 +25,8 @@
 //            once per block) the four u and o follow from numbers alone; a second pass updates
 //            the column for all four. The operands of the next 16 tokens travel to shared
 //            memory (cp.async) while the current 16 are worked on. Extra blocks write the
-//            convolution's inputs into the ring. (Keys of 128 values and longer portions: 32 tokens at a
-//            time by two kernels, gated_delta_chunks.cuh.)
+//            convolution's inputs into the ring. (Keys of 128 values: longer portions 32 tokens at a time
+//            by two kernels, gated_delta_chunks.cuh, shorter ones beside them.)
 //   finish   per (token, head): o / rms(o) * weight * silu(gate), in the compute type.
 // A step of single tokens runs one kernel, a block per (request, value head): the head's
 // matrix is asked for before the wait for the projection, the convolutions, norms and gates of
@@ -117,8 +117,8 @@ delta_prepare_kernel(const T* __restrict__ projected, const float* __restrict__ 
     griddep_launch();
 }
 
-// The same for keys of 128 values, convolutions of four taps and whole hundreds of 128 value channels:
-// runs of four tokens. A warp takes 128 channels (a query head and its key head one after the other, or
+// The same for keys of 128 values, convolutions of four taps and value channels that are a multiple of 128
+// over all heads: runs of four tokens. A warp takes 128 channels (a query head and its key head one after the other, or
 // values), a lane four neighbouring ones: seven loads of a run under way together, convolution weights
 // once a run. Bound by memory: 2,048 tokens of 4,096 channels, 16 MB in and 33 MB out: 30 us. (A block a
 // token, value by value: 53 us. Runs of eight need 160 registers and leave one block an SM: 59 us.)

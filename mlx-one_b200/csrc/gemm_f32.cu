@@ -429,7 +429,7 @@ int launch_skinny(const float* a, int lda, const float* w, int ldw, const float*
     const int groups = ceil_div_host(n, GROUP), slots = 2 * sm_count();
     int row_groups = ceil_div_host(groups, slots);
     row_groups = ceil_div_host(row_groups, side) * side;
-    // ... up to 32 KB of them at a time
+    // ... up to 32 KB of them at a time (64 KB where eight rows meet eight warps along K)
     const int depth = std::max(warps_k, std::min(ceil_div_host(sections, warps_k) * warps_k,
                                                  32 / MR / warps_k * warps_k));
     const auto bytes = [&](int g) {
@@ -453,9 +453,13 @@ int launch_skinny(const float* a, int lda, const float* w, int ldw, const float*
 bool aligned(const void* p, int to) { return reinterpret_cast<uintptr_t>(p) % to == 0; }
 
 // Which kernel. Up to 32 rows: w is what there is to read, and the streaming kernel reads it once per
-// eight rows, later times from L2 (32 rows, 1024 -> 1024 and 4608 -> 1024: 8 and 40 us against 22 and 78
-// us by tiles; 2048 -> 16384: 132 against 110 us). With 33 to 64 rows it would be behind at all but the
-// smallest matrices. One kernel for all, tiles of 64 x 64 walking K four values a thread at a time,
+// eight rows, later times from L2. Its time grows with every eight rows, the tiles' hardly does, so where the
+// two meet depends on the matrix. Us streamed / by tiles (with a cold L2) at 9 to 16, 17 to 24 and 25 to 32
+// rows: 1024 -> 1024 11 / 30, 13 / 30, 15 / 31; 8192 -> 2048 70 / 166, 96 / 177, 125 / 181; 1536 -> 4608 31 / 42,
+// 42 / 43, 48 / 44; 2048 -> 16384 80 / 95, 111 / 98, 140 / 102; 2048 -> 65536 282 / 291, 408 / 308, 537 / 320. One
+// line at 32 gains up to 150 us at the long narrow matrices and gives up to 217 away at the widest; a line
+// at 16 for matrices of more than about 6,000 rows would have both and is not drawn. With 33 to 64 rows the
+// streaming kernel would be behind at all but the smallest matrices. One kernel for all, tiles of 64 x 64 walking K four values a thread at a time,
 // took 134 us a product at one row of the 0.35 B shapes and 376 us at 1,200 rows beside decodes of the
 // 1.2 B ones. Now, us at 1 / 4 / 8 / 128 / 1,200 rows: 1024 -> 9216 (37.7 MB): 9.8 / 9.4 / 15 / 73 / 547;
 // 2048 -> 16384 (134 MB): 25 / 30 / 43 / 222 / 1932 (42 TFLOP/s); 8192 -> 2048: 18 / 26 / 43 / 158 / 1381.

@@ -286,11 +286,12 @@ class CudaOps:
 
     def _tcgen05(self, a, w, epilogue=0) -> bool:
         """Whether a[M, K] @ w[N, K]^T goes to the tcgen05 kernel. It needs 16-byte aligned
-        rows and at least 128 rows (its tiles are 128 x 256 and each persistent block walks
-        whole tiles), and it is chosen where it is faster than the library's product plus the
+        rows and at least 128 rows (its tiles are 128 x 256, or 128 x 192 where that takes no more
+        rounds over the SMs, and each persistent block walks whole tiles), and it is chosen where it is faster than the library's product plus the
         kernel that the library's product then needs: with the fused SwiGLU epilogue, which
         saves a pass over the widest activation (2048 rows: 100 us against 153 us; 512 rows: 35
-        against 41), when its tiles fill the SMs to 60 %. Plain products and products added into
+        against 41), when tiles of 128 x 256 fill the SMs to 60 % (measured with those; the
+        narrower ones only take over where the product is chosen by this rule). Plain products and products added into
         the residual stream go to the library, which is faster at every row count measured
         (2048 rows: in_proj 37.7 us against 45.3, qkv 20.7 against 30.8, out_proj 14.8 against
         24.8 with the residual epilogue, w2 47 against 62; 8192 rows: 142 / 73 / 49 / 181 us
@@ -1624,8 +1625,9 @@ class CudaOps:
         """Attention of every token over its request's pages. ``keep_first``: behind a window the
         first ``keep_first`` positions of a sequence stay visible. bfloat16 with a head size that
         is a multiple of 16 up to 128 runs on tensor cores: the split-key decode kernel when
-        every request brings one token, else the prefill kernel. Everything else (float32,
-        other head sizes) runs the general kernel. ``score_cap`` c (0: none): scores s become c
+        every request brings one token, else the prefill kernel. float32 with heads of 32, 64 or
+        128 values and every earlier key visible runs the 32-bit kernel (``_attention_f32``),
+        everything else the general one. ``score_cap`` c (0: none): scores s become c
         tanh(s / c); ``slopes`` (float32 [heads] or None): then they lose slope * (query's position
         - key's); ``least_slope`` is their minimum on the host."""
         if score_cap or slopes is not None:
