@@ -75,6 +75,10 @@ class CudaOps:
         # against 0.67 ms, batch 16 0.95 against 0.89 ms. So up to `fused_norm_max_rows` rows.
         self.fused_norms = True
         self.fused_norm_max_rows = 6
+        # 32-bit products of more rows than this on the tensor cores, each value cut into three bfloat16
+        # parts (csrc/gemm_f32_tcgen05.cu). Up to here all kernels add a row up in the same order.
+        self.f32_split = True
+        self.f32_split_rows = 130
         self.tcgen05_min_rows = 128
         self.tcgen05_attention = True     # prefill attention with tcgen05 where it takes the geometry
         # ... and with the keys of its few items cut into parts when a launch has fewer items than SMs
@@ -359,6 +363,10 @@ class CudaOps:
                    _c_void_p(_ptr(w)), _c_void_p(_ptr(bias)), _c_void_p(_ptr(out)), _c_int(ldo),
                    _c_int(a.shape[0]), _c_int(w.shape[0]), _c_int(a.shape[1]), _c_int(epilogue))
 
+    def _f32_split(self, a, w) -> bool:
+        return (self.f32_split and a.shape[0] > self.f32_split_rows and a.shape[1] % 8 == 0
+                and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
     def linear(self, a, w, bias=None, out_dtype=None):
         """a[M, K] @ w[N, K]^T (+ bias[N], float32). ``out_dtype``: a's dtype, or float32."""
         if isinstance(a, NormedInput):
@@ -375,6 +383,11 @@ class CudaOps:
             self._need_rows(a, torch.float32, "a")
             self._need(w, torch.float32, "w")
             out = torch.empty((m, n), dtype=torch.float32, device=self.device)
+            if self._f32_split(a, w):
+                self._call("mlxone_gemm_f32_split", _c_void_p(_ptr(a)), _c_int(max(a.stride(0), k)),
+                           _c_void_p(_ptr(w)), _c_int(k), _c_void_p(_ptr(bias)), _c_void_p(_ptr(out)), _c_int(n),
+                           _c_int(m), _c_int(n), _c_int(k), _c_void_p(_ptr(self.error_flag)))
+                return out
             self._call("mlxone_gemm_f32", _c_void_p(_ptr(a)), _c_int(max(a.stride(0), k)), _c_void_p(_ptr(w)),
                        _c_int(k), _c_void_p(_ptr(bias)), _c_void_p(_ptr(out)), _c_int(n),
                        _c_int(m), _c_int(n), _c_int(k))
