@@ -325,47 +325,50 @@ __global__ void swiglu_kernel(const T* __restrict__ gate_up, T* __restrict__ out
     out[i] = from_float<T>(gate / (1.f + expf(-gate)) * up);
 }
 
-// The same for bfloat16 with width % 8 == 0: eight neighbouring values a thread, 16-byte loads.
-__global__ void swiglu_wide_kernel(const __nv_bfloat16* __restrict__ gate_up,
-                                   __nv_bfloat16* __restrict__ out, int width, long long groups) {
+// The same where 16-byte pieces do not straddle rows: a piece a thread (four 32-bit or eight bfloat16
+// values). Bound by memory; a thread finds its row by a 32-bit division (by one of 64 bits for every single
+// value above).
+template <typename T>
+__global__ void swiglu_pieces_kernel(const T* __restrict__ gate_up, T* __restrict__ out, unsigned per_row,
+                                     unsigned pieces) {
+    constexpr int N = 16 / sizeof(T);
     griddep_launch();
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= pieces) return;
+    const unsigned t = i / per_row;
     griddep_wait();
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= groups) return;
-    const int per_row = width / 8;
-    const long long t = i / per_row;
-    const int f = (int)(i - t * per_row) * 8;
-    const uint4 g = *reinterpret_cast<const uint4*>(gate_up + t * 2 * width + f);
-    const uint4 u = *reinterpret_cast<const uint4*>(gate_up + t * 2 * width + width + f);
-    const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&g);
-    const __nv_bfloat162* up = reinterpret_cast<const __nv_bfloat162*>(&u);
-    uint4 packed;
-    __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&packed);
+    const uint4* from = reinterpret_cast<const uint4*>(settled(gate_up)) + (size_t)t * per_row + i;
+    const uint4 g = from[0], u = from[per_row];
+    const T *gates = reinterpret_cast<const T*>(&g), *ups = reinterpret_cast<const T*>(&u);
+    uint4 result;
+    T* values = reinterpret_cast<T*>(&result);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float g0 = __low2float(gp[k]), g1 = __high2float(gp[k]);
-        q[k] = __floats2bfloat162_rn(g0 / (1.f + expf(-g0)) * __low2float(up[k]),
-                                     g1 / (1.f + expf(-g1)) * __high2float(up[k]));
+    for (int k = 0; k < N; ++k) {
+        const float gate = to_float<T>(gates[k]);
+        values[k] = from_float<T>(gate / (1.f + expf(-gate)) * to_float<T>(ups[k]));
     }
-    *reinterpret_cast<uint4*>(out + t * width + f) = packed;
+    reinterpret_cast<uint4*>(out)[i] = result;
+}
+
+template <typename T>
+static void launch_swiglu(const void* gate_up, void* out, int rows, int width, cudaStream_t stream) {
+    constexpr int N = 16 / sizeof(T);
+    const long long total = (long long)rows * width;
+    if (width % N == 0 && total / N < (1ll << 31) &&
+        ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
+        launch_kernel(swiglu_pieces_kernel<T>, dim3(ceil_div_host(total / N, 256)), dim3(256), 0, stream, true,
+                      (const T*)gate_up, (T*)out, (unsigned)(width / N), (unsigned)(total / N));
+    else
+        launch_kernel(swiglu_kernel<T>, dim3(ceil_div_host(total, 256)), dim3(256), 0, stream, true,
+                      (const T*)gate_up, (T*)out, width, total);
 }
 
 MLXONE_API int mlxone_swiglu(const void* gate_up, void* out, int rows, int width, int dtype,
                              cudaStream_t stream) {
     if (rows == 0) return 0;
     MLXONE_REQUIRE(rows > 0 && width > 0, "swiglu: bad sizes");
-    const long long total = (long long)rows * width;
-    const int blocks = ceil_div_host(total, 256);
-    if (dtype == MLXONE_BF16 && width % 8 == 0 && (reinterpret_cast<uintptr_t>(gate_up) & 15) == 0 &&
-        (reinterpret_cast<uintptr_t>(out) & 15) == 0)
-        launch_kernel(swiglu_wide_kernel, dim3(ceil_div_host(total / 8, 256)), dim3(256), 0, stream,
-                      true, (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, width, total / 8);
-    else if (dtype == MLXONE_BF16)
-        launch_kernel(swiglu_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, true,
-                      (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, width, total);
-    else
-        launch_kernel(swiglu_kernel<float>, dim3(blocks), dim3(256), 0, stream, true,
-                      (const float*)gate_up, (float*)out, width, total);
+    if (dtype == MLXONE_BF16) launch_swiglu<__nv_bfloat16>(gate_up, out, rows, width, stream);
+    else launch_swiglu<float>(gate_up, out, rows, width, stream);
     MLXONE_LAUNCH_CHECK("swiglu");
     return 0;
 }
