@@ -811,7 +811,7 @@ int launch_delta(const void* projected, const float* conv, const float* a_log, c
                       (const float*)kq, (const T*)projected, state, slots, request_start, history, o, chunks,
                       sizes, requests, lead, chunk_from, places, write, ld);
         MLXONE_LAUNCH_CHECK("gated delta rule (chunks)");
-        launch_kernel(delta_walk_kernel<T>, dim3(V / DC_COLUMNS, H + 1, requests - lead), dim3(DC_WALK_THREADS),
+        launch_kernel(delta_walk_kernel<T>, dim3(V / DC_COLUMNS, H + 1, requests - lead), dim3(DC_THREADS),
                       DC_WALK_SHARED, stream, true, (const float*)q, (const float*)k, (const float*)v,
                       (const float*)chunks, (const T*)projected, state, slots, request_start, history, o,
                       sizes, lead, chunk_from, write, ld);

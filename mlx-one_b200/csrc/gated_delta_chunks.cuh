@@ -194,26 +194,28 @@ __device__ __forceinline__ void prepare_chunk(const float* q_in, const float* k_
 
 // ------------------------------------------------------------------ the walk
 // Grid (tiles of 16 columns of S, heads + 1, requests behind the first `lead`), of which those of fewer than
-// `chunk_from` tokens are the scan's; blocks with blockIdx.y == heads write the convolution's inputs into the
-// ring. S lies in shared memory and in the registers of the threads that update it. Bound by the chain from a
-// chunk's S to the next one's: S^T k, T diag(beta) r, the update. Eight warps do this and nothing else; the
-// outputs (S^T q, P T diag(beta) r) and the copies are eight other warps', beside it. (One group of eight warps
-// for all of it: 175 us for 2,048 tokens of 16 heads, 2.7 us a chunk. Tiles of 8 columns and twice the blocks
-// were 5 to 10 % slower, for 4 heads too.) Each product is 32 rows by 16 columns, a lane takes 4 x 4 outputs, a
-// warp an eighth of the sum (16 values of a key, 4 tokens), and the eighths are added up in order.
+// `chunk_from` tokens are the scan's; blocks with blockIdx.y == heads write the convolution's inputs into the ring. S lies in shared memory (and in the registers of the 128 threads
+// that update it). [k; q] S and [T diag(beta); P T diag(beta)] r are products of 64 rows by 16 columns: a
+// lane takes 8 x 4 outputs, a warp an eighth of the sum (16 values of a key, 4 tokens), and the eighths
+// are added up in order. Bound by the chain of products, barriers and reads of shared memory of a chunk
+// (2.6 us; 56 % of the SMs' shared memory reads, 40 % of their FMAs): tiles of 8 columns and twice the
+// blocks were 5 to 10 % slower, for 4 heads too. While half the warps update S the other half asks for the
+// chunk after next. 2,048 tokens of 16 heads: 170 us (530 by the scan of four tokens at a time).
 constexpr int DC_BUFFERS = 3;
 constexpr int DC_BUFFER = 2 * DC * DC_PITCH + DC * DC_COLUMNS + 2 * DC * DC_SMALL + 2 * DC;
-constexpr int DC_GROUP = 256, DC_WALK_THREADS = 2 * DC_GROUP;
 constexpr size_t DC_WALK_SHARED =
-    sizeof(float) * ((size_t)DC_BUFFERS * DC_BUFFER + DC_KEY * DC_COLUMNS + 2 * 8 * DC * DC_COLUMNS + 2 * DC * DC_COLUMNS);
+    sizeof(float) * ((size_t)DC_BUFFERS * DC_BUFFER + DC_KEY * DC_COLUMNS + 8 * 2 * DC * DC_COLUMNS + 2 * DC * DC_COLUMNS);
 
-// acc (rows lane / 4 + 8 i, columns 4 (lane % 4) .. + 3) += x[32 rows, 4 STEPS columns] * y[4 STEPS rows, 16
-// columns]. LOWER: x is zero above the diagonal (`column`: where its first column here stands), and what
-// stands there meets nothing of y.
+// part[warp][64][16] = x[64 rows, 4 STEPS columns from e0] * y[4 STEPS rows, 16 columns]. LOWER: x is two
+// matrices of 32 rows that are zero above the diagonal (`column`: where its first column here stands), and
+// what stands there meets nothing of y.
 template <int STEPS, bool LOWER = false>
-__device__ __forceinline__ void chunk_product(FloatPair (&acc)[4][2], const float* x, int pitch, const float* y,
+__device__ __forceinline__ void chunk_product(const float* x, int pitch, const float* y, float* part,
                                               int column = 0) {
     const int lane = threadIdx.x & 31, rg = lane >> 2, cg = lane & 3;
+    FloatPair acc[8][2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = 0;
 #pragma unroll
     for (int step = 0; step < STEPS; ++step) {
         ulonglong2 b[4];
@@ -221,51 +223,35 @@ __device__ __forceinline__ void chunk_product(FloatPair (&acc)[4][2], const floa
         for (int e = 0; e < 4; ++e)
             b[e] = *reinterpret_cast<const ulonglong2*>(y + (step * 4 + e) * DC_COLUMNS + cg * 4);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 8; ++i) {
             const float4 v = *reinterpret_cast<const float4*>(x + (rg + 8 * i) * pitch + step * 4);
             const float values[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                if (LOWER && column + step * 4 + e > rg + 8 * i) continue;
+                if (LOWER && column + step * 4 + e > (rg + 8 * i) % DC) continue;
                 const FloatPair f = pair_of(values[e]);
                 accumulate_pair(acc[i][0], f, b[e].x);
                 accumulate_pair(acc[i][1], f, b[e].y);
             }
         }
     }
-}
-// part[32][16] = acc
-__device__ __forceinline__ void store_part(float* part, const FloatPair (&acc)[4][2]) {
-    const int lane = threadIdx.x & 31, rg = lane >> 2, cg = lane & 3;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 8; ++i)
         *reinterpret_cast<float4*>(part + (rg + 8 * i) * DC_COLUMNS + cg * 4) = quad_of(acc[i][0], acc[i][1]);
-}
-// the eighths of two outputs added up
-__device__ __forceinline__ float2 gather_parts(const float* part, int at) {
-    float2 sum = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-        const float2 v = *reinterpret_cast<const float2*>(part + w * DC * DC_COLUMNS + at);
-        sum.x += v.x; sum.y += v.y;
-    }
-    return sum;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(DC_WALK_THREADS)
+__global__ void __launch_bounds__(DC_THREADS)
 delta_walk_kernel(const float* q_in, const float* k_in, const float* v_in, const float* chunks,
                   const T* __restrict__ projected, float* state, const int* __restrict__ slots,
                   const int* __restrict__ request_start, const int* __restrict__ history, float* out,
                   DeltaSizes sizes, int lead, int chunk_from, int write, int ld) {
     extern __shared__ __align__(16) float shared[];
     float* matrix_s = shared + DC_BUFFERS * DC_BUFFER;       // S [128][16]
-    float* parts = matrix_s + DC_KEY * DC_COLUMNS;           // [2 groups of warps][8][32][16]
-    float* rest = parts + 2 * 8 * DC * DC_COLUMNS;           // r [32][16]
+    float* part = matrix_s + DC_KEY * DC_COLUMNS;            // [8][64][16]
+    float* rest = part + 8 * 2 * DC * DC_COLUMNS;            // r [32][16]
     float* moved = rest + DC * DC_COLUMNS;                   // D(32, t) u_t [32][16]
-    // the chain's warps are the first eight
-    const int tid = threadIdx.x % DC_GROUP, warp = tid >> 5, r = lead + blockIdx.z;
-    const bool chain = threadIdx.x < DC_GROUP;
+    const int tid = threadIdx.x, warp = tid >> 5, r = lead + blockIdx.z;
     griddep_wait();
     const int first = request_start[r], last = request_start[r + 1];
     if (last - first < chunk_from) return;
@@ -277,141 +263,141 @@ delta_walk_kernel(const float* q_in, const float* k_in, const float* v_in, const
         const int channels = sizes.channels(), taps = sizes.taps;
         const int n = last - first, kept = min(n, taps);
         float* ring = slot + sizes.matrices();
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < channels; c += gridDim.x * blockDim.x)
+        for (int c = blockIdx.x * blockDim.x + tid; c < channels; c += gridDim.x * blockDim.x)
             for (int index = n - kept; index < n; ++index)
                 ring[(size_t)((history[r] + index) % taps) * channels + c] =
                     to_float<T>(projected[(size_t)(first + index) * ld + c]);
         return;
     }
     const int h = blockIdx.y, g = h / (H / G), column0 = blockIdx.x * DC_COLUMNS;
-    // the chunk's operands into its buffer, by the outputs' warps; a group of copies even where there is no
-    // such chunk
-    auto fetch = [&](int chunk) {
+    // the chunk's operands into its buffer, by `count_of` threads of which this is number `me`; a group of
+    // copies even where there is no such chunk
+    auto fetch = [&](int chunk, int me, int count_of) {
         if (first + chunk * DC >= last) { copy_commit(); return; }
         float* to = shared + chunk % DC_BUFFERS * DC_BUFFER;
         const int base = first + chunk * DC, count = min(DC, last - base);
-        for (int i = tid; i < 2 * DC * (DC_KEY / 4); i += DC_GROUP) {
+        for (int i = me; i < 2 * DC * (DC_KEY / 4); i += count_of) {
             const int row = i / (DC_KEY / 4), e = i % (DC_KEY / 4) * 4, t = row % DC;
             copy_or_zero_16(to + row * DC_PITCH + e,
                             (row < DC ? k_in : q_in) + ((size_t)(base + min(t, count - 1)) * G + g) * DC_KEY + e,
                             t < count);
         }
         to += 2 * DC * DC_PITCH;
-        if (tid < DC * (DC_COLUMNS / 4)) {
-            const int t = tid / (DC_COLUMNS / 4), c = tid % (DC_COLUMNS / 4) * 4;
+        if (me < DC * (DC_COLUMNS / 4)) {
+            const int t = me / (DC_COLUMNS / 4), c = me % (DC_COLUMNS / 4) * 4;
             copy_or_zero_16(to + t * DC_COLUMNS + c,
                             v_in + ((size_t)(base + min(t, count - 1)) * H + h) * V + column0 + c, t < count);
         }
         to += DC * DC_COLUMNS;
         const float* from = chunks + ((size_t)(first_chunk(first, r, lead) + chunk) * H + h) * DC_VALUES;
-        for (int i = tid; i < 2 * DC * (DC / 4); i += DC_GROUP) {
+        for (int i = me; i < 2 * DC * (DC / 4); i += count_of) {
             const int row = i / (DC / 4), e = i % (DC / 4) * 4;
             copy_or_zero_16(to + row * DC_SMALL + e, from + row * DC + e, true);
         }
         to += 2 * DC * DC_SMALL;
-        if (tid < 2 * DC / 4) copy_or_zero_16(to + tid * 4, from + 2 * DC * DC + tid * 4, true);
+        if (me < 2 * DC / 4) copy_or_zero_16(to + me * 4, from + 2 * DC * DC + me * 4, true);
         copy_commit();
     };
     const int total = (last - first + DC - 1) / DC;
-    // S: thread t of the chain keeps rows 2 (t / 4) and + 1 of columns 4 (t % 4) .. + 3
-    const int own_row = tid / 4 * 2, own_column = tid % 4 * 4;
+    fetch(0, tid, DC_THREADS);
+    fetch(1, tid, DC_THREADS);
+    // S: thread t < 128 keeps rows 4 (t / 4) .. + 3 of columns 4 (t % 4) .. + 3
+    const int own_row = tid / 4 * 4, own_column = tid % 4 * 4;
     float* matrix = slot + (size_t)h * DC_KEY * V + column0;
-    FloatPair S[2][2];
-    if (chain) {
+    FloatPair S[4][2];
+    if (tid < 128) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 4; ++i) {
             const float* from = matrix + (size_t)(own_row + i) * V + own_column;
             S[i][0] = pair_of(from[0], from[1]);
             S[i][1] = pair_of(from[2], from[3]);
             *reinterpret_cast<float4*>(matrix_s + (own_row + i) * DC_COLUMNS + own_column) =
                 quad_of(S[i][0], S[i][1]);
         }
-    } else {
-        fetch(0);
-        fetch(1);
-        copy_wait_for<1>();
     }
-    __syncthreads();
-    float* part = parts + (chain ? 0 : 8 * DC * DC_COLUMNS);
-    float* mine = part + warp * DC * DC_COLUMNS;
-    // barrier of this group of warps
-    auto meet = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(chain ? 1 : 2), "n"(DC_GROUP) : "memory"); };
-    const int row = tid / 8, at = tid * 2;                   // two outputs of 32 x 16: row, place
+    // sums of the eighths: thread t adds up four columns of row t / 4
+    const int row = tid / 4;
+    auto gather = [&]() {
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            const float4 v =
+                *reinterpret_cast<const float4*>(part + (w * 2 * DC + row) * DC_COLUMNS + own_column);
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+        }
+        return sum;
+    };
     for (int chunk = 0; chunk < total; ++chunk) {
         const float* kq = shared + chunk % DC_BUFFERS * DC_BUFFER;
         const float* vs = kq + 2 * DC * DC_PITCH;
         const float* small = vs + DC * DC_COLUMNS;
         const float* decays = small + 2 * DC * DC_SMALL;     // G_t, D(32, t)
-        FloatPair acc[4][2];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0;
-        if (chain) {
-            chunk_product<4>(acc, kq + warp * 16, DC_PITCH, matrix_s + warp * 16 * DC_COLUMNS);
-            store_part(mine, acc);
-            meet();
-            const float2 with_k = gather_parts(part, at);
-            const float before = decays[row];
-            const float2 v = *reinterpret_cast<const float2*>(vs + at);
-            const float2 left = make_float2(fmaf(-before, with_k.x, v.x), fmaf(-before, with_k.y, v.y));
-            *reinterpret_cast<float2*>(rest + at) = left;
-            // (zero times an infinity or NaN of a later token would reach the tokens before it)
-            const bool finite = __syncthreads_and(isfinite(left.x) && isfinite(left.y));
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0;
-            if (finite) chunk_product<1>(acc, small + warp * 4, DC_SMALL, rest + warp * 4 * DC_COLUMNS);
-            else chunk_product<1, true>(acc, small + warp * 4, DC_SMALL, rest + warp * 4 * DC_COLUMNS, warp * 4);
-            store_part(mine, acc);
-            meet();
-            const float2 u = gather_parts(part, at);
+        copy_wait_for<1>();                                  // (the chunk behind this one may be under way)
+        __syncthreads();
+        chunk_product<4>(kq + warp * 16, DC_PITCH, matrix_s + warp * 16 * DC_COLUMNS,
+                         part + warp * 2 * DC * DC_COLUMNS);
+        __syncthreads();
+        float4 with_q = gather();                            // (rows of k: becomes r)
+        const float before = decays[row % DC];
+        bool finite = true;
+        if (row < DC) {
+            const float4 v = *reinterpret_cast<const float4*>(vs + row * DC_COLUMNS + own_column);
+            const float4 r = make_float4(fmaf(-before, with_q.x, v.x), fmaf(-before, with_q.y, v.y),
+                                         fmaf(-before, with_q.z, v.z), fmaf(-before, with_q.w, v.w));
+            finite = isfinite(r.x) && isfinite(r.y) && isfinite(r.z) && isfinite(r.w);
+            *reinterpret_cast<float4*>(rest + row * DC_COLUMNS + own_column) = r;
+        }
+        // (zero times an infinity or NaN of a later token would reach the tokens before it)
+        if (__syncthreads_and(finite))
+            chunk_product<1>(small + warp * 4, DC_SMALL, rest + warp * 4 * DC_COLUMNS,
+                             part + warp * 2 * DC * DC_COLUMNS);
+        else
+            chunk_product<1, true>(small + warp * 4, DC_SMALL, rest + warp * 4 * DC_COLUMNS,
+                                   part + warp * 2 * DC * DC_COLUMNS, warp * 4);
+        __syncthreads();
+        const float4 sum = gather();
+        if (row < DC) {
             const float after = decays[DC + row];
-            *reinterpret_cast<float2*>(moved + at) = make_float2(after * u.x, after * u.y);
-            meet();
+            *reinterpret_cast<float4*>(moved + row * DC_COLUMNS + own_column) =
+                make_float4(after * sum.x, after * sum.y, after * sum.z, after * sum.w);
+        } else if (first + chunk * DC + row - DC < last) {
+            float* to = out + ((size_t)(first + chunk * DC + row - DC) * H + h) * V + column0 + own_column;
+            *reinterpret_cast<float4*>(to) =
+                make_float4(fmaf(before, with_q.x, sum.x), fmaf(before, with_q.y, sum.y),
+                            fmaf(before, with_q.z, sum.z), fmaf(before, with_q.w, sum.w));
+        }
+        __syncthreads();
+        if (tid < 128) {
+            // (half the warps, the other half asks for the chunk after next meanwhile)
             const FloatPair whole = pair_of(decays[DC - 1]);
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int j = 0; j < 2; ++j) S[i][j] = mul_pair(S[i][j], whole);
 #pragma unroll 8
             for (int t = 0; t < DC; ++t) {
-                const float2 k = *reinterpret_cast<const float2*>(kq + t * DC_PITCH + own_row);
-                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(moved + t * DC_COLUMNS + own_column);
-                const FloatPair ks[2] = {pair_of(k.x), pair_of(k.y)};
+                const float4 k = *reinterpret_cast<const float4*>(kq + t * DC_PITCH + own_row);
+                const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(moved + t * DC_COLUMNS + own_column);
+                const FloatPair ks[4] = {pair_of(k.x), pair_of(k.y), pair_of(k.z), pair_of(k.w)};
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    accumulate_pair(S[i][0], ks[i], x.x);
-                    accumulate_pair(S[i][1], ks[i], x.y);
+                for (int i = 0; i < 4; ++i) {
+                    accumulate_pair(S[i][0], ks[i], u.x);
+                    accumulate_pair(S[i][1], ks[i], u.y);
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
+            for (int i = 0; i < 4; ++i)
                 *reinterpret_cast<float4*>(matrix_s + (own_row + i) * DC_COLUMNS + own_column) =
                     quad_of(S[i][0], S[i][1]);
+            copy_commit();                                   // (groups are counted thread by thread)
         } else {
-            chunk_product<4>(acc, kq + DC * DC_PITCH + warp * 16, DC_PITCH, matrix_s + warp * 16 * DC_COLUMNS);
-            fetch(chunk + 2);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const FloatPair before = pair_of(decays[(threadIdx.x & 31) / 4 + 8 * i]);
-                acc[i][0] = mul_pair(acc[i][0], before);
-                acc[i][1] = mul_pair(acc[i][1], before);
-            }
-            const float* p = small + DC * DC_SMALL + warp * 4;
-            if (__syncthreads_and(true)) chunk_product<1>(acc, p, DC_SMALL, rest + warp * 4 * DC_COLUMNS);
-            else chunk_product<1, true>(acc, p, DC_SMALL, rest + warp * 4 * DC_COLUMNS, warp * 4);
-            store_part(mine, acc);
-            meet();
-            const float2 o = gather_parts(part, at);
-            if (first + chunk * DC + row < last)
-                *reinterpret_cast<float2*>(out + ((size_t)(first + chunk * DC + row) * H + h) * V + column0 +
-                                           at % DC_COLUMNS) = o;
-            copy_wait_for<1>();                              // (the next chunk; the one behind it may be under way)
+            fetch(chunk + 2, tid - 128, 128);
         }
-        __syncthreads();
     }
     griddep_launch();
-    if (write && chain) {
+    if (write && tid < 128) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 4; ++i) {
             const float4 v = quad_of(S[i][0], S[i][1]);
             float* to = matrix + (size_t)(own_row + i) * V + own_column;
             to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w;
