@@ -9,8 +9,9 @@
 //            ring of stages guarded by mbarriers;
 //   warp 1   allocates tensor memory and one thread issues tcgen05.mma (M = 128, N = BN,
 //            K = 16, four per stage), releasing each stage with tcgen05.commit;
-//   warps 2-5  the epilogue: each reads its quarter of the accumulator's 128 lanes with
-//            tcgen05.ld, 32 columns at a time, and writes the result.
+//   warps 2-9  the epilogue: each reads its quarter of the accumulator's 128 lanes with
+//            tcgen05.ld, every other 32 columns, and writes the result. (With four warps a gated
+//            tile's epilogue took 6.8 us, more than its products for K = 1,024.)
 // Both operands are K-major, so no transposition is needed anywhere.
 //
 // Epilogues: store bfloat16 (+ bias); SwiGLU (the w tile is 128 gate rows followed by the 128
@@ -31,7 +32,8 @@ constexpr int BK = 64;                 // 64 bf16 = 128 bytes: one swizzle row
 constexpr int WIDE_STAGES = 4;         // 128 x 256 tiles: 4 x 48 KB
 constexpr int MIDDLE_STAGES = 5;       // 128 x 192 tiles: 5 x 40 KB
 constexpr int NARROW_STAGES = 6;       // 128 x 128 tiles: 6 x 32 KB
-constexpr int THREADS = 192;           // producer warp, mma warp, four epilogue warps
+constexpr int PAIR_STAGES = 6;         // 256 x 256 tiles of two blocks: 6 x 32 KB in each
+constexpr int EPILOGUE_WARPS = 8, THREADS = 64 + 32 * EPILOGUE_WARPS;  // and a producer warp, an mma warp
 constexpr int WAIT_LIMIT = 1 << 24;    // polls before a wait gives up
 constexpr int ERROR_WAIT = 9;
 
@@ -82,6 +84,28 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 
+// The same for a pair of blocks: the barrier may be the other block's.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y,
+                                                 uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, "
+        "{%3, %4}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
+        : "memory");
+}
+__device__ __forceinline__ uint32_t address_in(uint32_t address, int rank) {
+    uint32_t there;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(address), "r"(rank));
+    return there;
+}
+__device__ __forceinline__ void barrier_arrive_in(uint32_t bar, int rank) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(address_in(bar, rank))
+                 : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
 // ------------------------------------------------------------------ tcgen05
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_shared, int columns) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_shared),
@@ -107,6 +131,28 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
     asm volatile(
         "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
+        : "memory");
+}
+// ... of a pair of blocks, which the first one issues: 256 rows of A and of B, half of each in either block's
+// shared memory, the halves of the rows of D in either block's tensor memory
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_shared, int columns) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_shared),
+                 "r"(columns));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+}
+__device__ __forceinline__ void tmem_free_pair(uint32_t address, int columns) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(address), "r"(columns));
+}
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void mma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                              uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
         : "memory");
 }
@@ -146,10 +192,23 @@ __host__ __device__ constexpr uint32_t instruction_descriptor(int m, int n) {
            ((uint32_t)(m >> 4) << 24);
 }
 
+__device__ __forceinline__ float exponential(float x) {       // 2^x
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float reciprocal(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // Two accumulators of BN columns; tensor memory is given out in powers of two.
 __host__ __device__ constexpr int tmem_columns(int bn) { return bn <= 128 ? 256 : 512; }
 
-template <int BN, int EPILOGUE, int STAGES>
+// PAIR: blocks work in clusters of two on tiles of 256 x BN: each brings its 128 rows of `a` and half of the
+// tile's rows of w (SwiGLU: the gate's or the up half) and finishes its own 128 rows.
+template <int BN, int EPILOGUE, int STAGES, bool PAIR>
 __global__ void __launch_bounds__(THREADS)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     const __grid_constant__ CUtensorMap map_w, const float* __restrict__ bias,
@@ -162,7 +221,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     // matrices stacked in `w`: a product per expert in one launch. `out_limit` is the number of
     // output columns (the width of one expert's result). `clamp` (SWIGLU): positive: the limit of the
     // clamped gated form (mlxone_clamped) instead of silu(gate) * up.
-    constexpr int A_BYTES = BM * BK * 2, W_BYTES = BN * BK * 2;
+    constexpr int A_BYTES = BM * BK * 2, W_BYTES = BN * BK * 2 / (PAIR ? 2 : 1);
+    constexpr int TILE_M = PAIR ? 2 * BM : BM;
     constexpr int OUT_COLUMNS = EPILOGUE == SWIGLU ? BN / 2 : BN;
     extern __shared__ unsigned char shared_raw[];
     // full[s], empty[s] per stage; ready[b], drained[b] per accumulator buffer
@@ -172,6 +232,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     const uint32_t tiles = (shared_address(shared_raw) + 1023u) & ~1023u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k_tiles = (k + BK - 1) / BK;
+    const int rank = PAIR ? blockIdx.x & 1 : 0;
+    const int first_tile = PAIR ? blockIdx.x >> 1 : blockIdx.x, tile_step = PAIR ? gridDim.x >> 1 : gridDim.x;
     auto full = [&](int s) { return shared_address(&barriers[s]); };
     auto empty = [&](int s) { return shared_address(&barriers[STAGES + s]); };
     auto ready = [&](int b) { return shared_address(&barriers[2 * STAGES + b]); };
@@ -184,13 +246,18 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         }
         for (int b = 0; b < 2; ++b) {
             barrier_init(ready(b), 1);
-            barrier_init(drained(b), 4);               // the four epilogue warps
+            barrier_init(drained(b), (PAIR ? 2 : 1) * EPILOGUE_WARPS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(shared_address(&tmem_base_slot), tmem_columns(BN));
+    if (warp == 1) {
+        if (PAIR) tmem_alloc_pair(shared_address(&tmem_base_slot), tmem_columns(BN));
+        else tmem_alloc(shared_address(&tmem_base_slot), tmem_columns(BN));
+    }
     fence_before_sync();
+    __syncwarp();
+    if (PAIR) cluster_barrier();             // (both blocks' barriers are there before either is used)
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
@@ -202,8 +269,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         if (lane == 0) {
             int step = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-                const int tile_m = (tile % tiles_m) * BM;
+            for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
+                const int tile_m = (tile % tiles_m) * TILE_M + rank * BM;
                 int tile_n = (tile / tiles_m) * OUT_COLUMNS, w_column = 0;
                 if (groups != nullptr) {
                     const int2 group = groups[tile % tiles_m];
@@ -215,8 +282,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     const int s = step % STAGES;
                     ok = barrier_wait(empty(s), ((step / STAGES) & 1) ^ 1, error_flag);
                     if (!ok) break;
-                    barrier_expect(full(s), A_BYTES + W_BYTES);
                     const uint32_t a_tile = tiles + s * (A_BYTES + W_BYTES);
+                    if (PAIR) {
+                        // both blocks' copies count on the first one's barrier
+                        if (rank == 0) barrier_expect(full(s), 2 * (A_BYTES + W_BYTES));
+                        const uint32_t bar = address_in(full(s), 0);
+                        const int w_row = tile_n + (EPILOGUE == SWIGLU ? rank * up_offset : rank * (BN / 2));
+                        tma_load_2d_pair(a_tile, &map_a, kt * BK, tile_m, bar);
+                        tma_load_2d_pair(a_tile + A_BYTES, &map_w, kt * BK, w_row, bar);
+                        continue;
+                    }
+                    barrier_expect(full(s), A_BYTES + W_BYTES);
                     tma_load_2d(a_tile, &map_a, kt * BK, tile_m, full(s));
                     tma_load_2d(a_tile + A_BYTES, &map_w, w_column + kt * BK, tile_n, full(s));
                     if (EPILOGUE == SWIGLU)
@@ -226,11 +302,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = instruction_descriptor(BM, BN);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = instruction_descriptor(TILE_M, BN);
             int step = 0, round = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+            for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
                 if (groups != nullptr && groups[tile % tiles_m].x < 0) continue;
                 const int buffer = round & 1;
                 // the epilogue must have read this buffer's previous tile
@@ -247,43 +323,56 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     const uint64_t a_desc = operand_descriptor(a_tile);
                     const uint64_t w_desc = operand_descriptor(a_tile + A_BYTES);
 #pragma unroll
-                    for (int kk = 0; kk < BK / 16; ++kk)   // 16 bf16 = 32 bytes = 2 address units
-                        mma_bf16(accumulator, a_desc + 2 * kk, w_desc + 2 * kk, idesc,
-                                 kt > 0 || kk > 0);
-                    mma_commit(empty(s));                  // the stage is free once these finish
+                    for (int kk = 0; kk < BK / 16; ++kk) { // 16 bf16 = 32 bytes = 2 address units
+                        if (PAIR) mma_bf16_pair(accumulator, a_desc + 2 * kk, w_desc + 2 * kk, idesc, kt > 0 || kk > 0);
+                        else mma_bf16(accumulator, a_desc + 2 * kk, w_desc + 2 * kk, idesc, kt > 0 || kk > 0);
+                    }
+                    // the stage is free once these finish
+                    if (PAIR) mma_commit_pair(empty(s));
+                    else mma_commit(empty(s));
                 }
-                if (ok) mma_commit(ready(buffer));
+                if (ok && PAIR) mma_commit_pair(ready(buffer));
+                if (ok && !PAIR) mma_commit(ready(buffer));
                 ++round;
             }
         }
     } else {
-        // epilogue warps 2..5 read the lane quarters 2, 3, 0, 1 (a warp may only touch its own).
+        // epilogue warps 2..9 read the lane quarters 2, 3, 0, 1, 2, ... (a warp may only touch its own).
         // A thread gets 32 columns of one row from tensor memory and writes them itself.
-        const int quarter = warp & 3;
+        const int quarter = warp & 3, side = (warp - 2) >> 2;
         float* turn = reinterpret_cast<float*>(shared_raw + (tiles - shared_address(shared_raw)) +
-                                               STAGES * (A_BYTES + W_BYTES)) + (warp - 2) * 32 * 33;
+                                               STAGES * (A_BYTES + W_BYTES)) + (warp - 2) * 32 * 17;
         const int limit = out_limit;
+        // SwiGLU without biases and limits, as it mostly is: a value costs six instructions, two of them of the
+        // unit that does sixteen a cycle
+        const bool plain_gate = bias == nullptr && !(clamp > 0.f);
         // whether every row of the output starts on a 16-byte boundary
         const bool whole_rows =
             stores_bf16(EPILOGUE)
                 ? (ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0)
                 : (ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0);
         int round = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
+        for (int tile = first_tile; tile < total_tiles; tile += tile_step) {
             if (groups != nullptr && groups[tile % tiles_m].x < 0) continue;
             const int buffer = round++ & 1;
-            const int tile_m = (tile % tiles_m) * BM;
+            const int tile_m = (tile % tiles_m) * TILE_M + rank * BM;
             const int tile_n = (tile / tiles_m) * OUT_COLUMNS;
             if (!barrier_wait(ready(buffer), ((round - 1) >> 1) & 1, error_flag)) break;
             fence_after_sync();
             const uint32_t accumulator = tmem_base + buffer * BN + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-            for (int c0 = 0; c0 < OUT_COLUMNS; c0 += 32) {
+            for (int c0 = 32 * side; c0 < OUT_COLUMNS; c0 += 64) {
                 float value[32];
                 tmem_load_32(accumulator + c0, value);
                 if (EPILOGUE == SWIGLU) {
                     float up[32];
                     tmem_load_32(accumulator + BN / 2 + c0, up);
+                    // (the result is rounded to bfloat16; the fast exponential and reciprocal are exact enough)
+                    if (plain_gate) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            value[i] = value[i] * reciprocal(1.f + exponential(value[i] * -1.4426950408889634f)) * up[i];
+                    } else {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
                         float gate = value[i], other = up[i];
@@ -297,8 +386,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                             other = fminf(fmaxf(other, -clamp), clamp) + 1.f;
                             steep = 1.702f;
                         }
-                        // the result is rounded to bfloat16; the fast exponential is exact enough
                         value[i] = __fdividef(gate, 1.f + __expf(-steep * gate)) * other;
+                    }
                     }
                 } else if (bias != nullptr) {
 #pragma unroll
@@ -312,11 +401,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                         value[i] = positive * positive;
                     }
                 }
-                if (c0 + 32 >= OUT_COLUMNS) {
+                if (c0 + 64 >= OUT_COLUMNS) {
                     // the last piece has left tensor memory: the buffer may be overwritten
                     fence_before_sync();
                     __syncwarp();
-                    if (lane == 0)
+                    if (lane == 0 && PAIR)
+                        barrier_arrive_in(drained(buffer), 0);
+                    else if (lane == 0)
                         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(drained(buffer))
                                      : "memory");
                 }
@@ -362,40 +453,51 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     continue;
                 }
                 // rows that 16-byte accesses cannot take, or the ragged last columns: the warp
-                // turns its 32 x 32 piece around in shared memory and writes a row at a time
-                __syncwarp();
-#pragma unroll
-                for (int i = 0; i < 32; ++i) turn[lane * 33 + i] = value[i];
-                __syncwarp();
-                const int column = tile_n + c0 + lane;
+                // turns its 32 x 32 piece around in shared memory, 16 columns at a time, and writes
+                // two rows at a time
                 const int row0 = tile_m + quarter * 32;
                 const int rows = min(32, m - row0);
-                if (column < limit && rows > 0) {
+#pragma unroll
+                for (int part = 0; part < 32; part += 16) {
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) turn[lane * 17 + i] = value[part + i];
+                    __syncwarp();
+                    const int column = tile_n + c0 + part + (lane & 15);
+                    if (column >= limit) continue;
                     const size_t at = (size_t)row0 * ldo + column;
+                    const float* from = turn + (lane & 15);
                     if (stores_bf16(EPILOGUE)) {
                         bf16* dst = reinterpret_cast<bf16*>(out) + at;
 #pragma unroll 8
-                        for (int r = 0; r < rows; ++r)
-                            dst[(size_t)r * ldo] = __float2bfloat16_rn(turn[r * 33 + lane]);
+                        for (int r = lane >> 4; r < rows; r += 2)
+                            dst[(size_t)r * ldo] = __float2bfloat16_rn(from[r * 17]);
                     } else if (EPILOGUE == ADD_RESIDUAL) {
                         float* dst = reinterpret_cast<float*>(out) + at;
                         // all loads first: they do not wait for one another
-                        float old[32];
+                        float old[16];
 #pragma unroll
-                        for (int r = 0; r < 32; ++r) old[r] = r < rows ? dst[(size_t)r * ldo] : 0.f;
+                        for (int i = 0; i < 16; ++i) {
+                            const int r = 2 * i + (lane >> 4);
+                            old[i] = r < rows ? dst[(size_t)r * ldo] : 0.f;
+                        }
 #pragma unroll
-                        for (int r = 0; r < 32; ++r)
-                            if (r < rows) dst[(size_t)r * ldo] = old[r] + turn[r * 33 + lane];
+                        for (int i = 0; i < 16; ++i) {
+                            const int r = 2 * i + (lane >> 4);
+                            if (r < rows) dst[(size_t)r * ldo] = old[i] + from[r * 17];
+                        }
                     } else {
                         float* dst = reinterpret_cast<float*>(out) + at;
 #pragma unroll 8
-                        for (int r = 0; r < rows; ++r) dst[(size_t)r * ldo] = turn[r * 33 + lane];
+                        for (int r = lane >> 4; r < rows; r += 2) dst[(size_t)r * ldo] = from[r * 17];
                     }
                 }
             }
         }
     }
     fence_before_sync();
+    __syncwarp();
+    if (PAIR) cluster_barrier();             // (the other block's copies and products end here too)
     __syncthreads();
     if (warp == 1) {
         fence_after_sync();
@@ -404,7 +506,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
             // shared memory before the block ends
             for (int i = 0; i < 1000; ++i) __nanosleep(1000);
         }
-        tmem_free(tmem_base, tmem_columns(BN));
+        if (PAIR) tmem_free_pair(tmem_base, tmem_columns(BN));
+        else tmem_free(tmem_base, tmem_columns(BN));
     }
 }
 
@@ -460,18 +563,18 @@ int sm_count() {
     return g_sm_count;
 }
 
-// How many tiles of 128 rows by `columns` an SM works through for a gated product.
-int gated_rounds(int m, int width, int columns) {
-    const long long tiles = (long long)((m + BM - 1) / BM) * ((width + columns - 1) / columns);
-    return (int)((tiles + sm_count() - 1) / sm_count());
+// How many tiles of 128 `blocks` rows by `columns` such a number of blocks works through for a gated product.
+int gated_rounds(int m, int width, int columns, int blocks) {
+    const long long tiles = (long long)((m + BM * blocks - 1) / (BM * blocks)) * ((width + columns - 1) / columns);
+    return ceil_div_host(tiles, sm_count() / blocks);
 }
 
-template <int BN, int EPILOGUE, int STAGES>
+template <int BN, int EPILOGUE, int STAGES, bool PAIR = false>
 int launch(const void* a, int lda, const void* w, const float* bias, void* out, int ldo, int m,
            int n, int k, int up_offset, int* error_flag, cudaStream_t stream,
            Grouping grouping = Grouping(), float clamp = 0.f) {
     CUtensorMap map_a, map_w;
-    const int w_box = EPILOGUE == SWIGLU ? BN / 2 : BN;
+    const int w_box = EPILOGUE == SWIGLU || PAIR ? BN / 2 : BN;
     const bool grouped = grouping.groups != nullptr;
     const bool mapped = grouped
         ? make_map(&map_w, w, grouping.w_rows, grouping.w_columns, grouping.w_ld, w_box)
@@ -482,20 +585,32 @@ int launch(const void* a, int lda, const void* w, const float* bias, void* out, 
     }
     const int out_columns = EPILOGUE == SWIGLU ? BN / 2 : BN;
     const int columns = grouped ? grouping.out_limit : EPILOGUE == SWIGLU ? up_offset : n;
-    const int tiles_m = (m + BM - 1) / BM;
+    const int tile_m = PAIR ? 2 * BM : BM, tiles_m = (m + tile_m - 1) / tile_m;
     const int total_tiles = tiles_m * ((columns + out_columns - 1) / out_columns);
-    const dim3 grid(total_tiles < sm_count() ? total_tiles : sm_count());
-    const size_t shared = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 1024 + 4 * 32 * 33 * 4;
-    auto kernel = gemm_tcgen05_kernel<BN, EPILOGUE, STAGES>;
+    const int workers = PAIR ? sm_count() / 2 : sm_count();
+    const dim3 grid((total_tiles < workers ? total_tiles : workers) * (PAIR ? 2 : 1));
+    const size_t shared = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2 / (PAIR ? 2 : 1)) + 1024 +
+                          EPILOGUE_WARPS * 32 * 17 * 4;
+    auto kernel = gemm_tcgen05_kernel<BN, EPILOGUE, STAGES, PAIR>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)shared);
     if (err != cudaSuccess) {
         mlxone_set_error("gemm_tcgen05: %s", cudaGetErrorString(err));
         return 2;
     }
-    kernel<<<grid, THREADS, shared, stream>>>(map_a, map_w, bias, out, ldo, m, n, k, up_offset,
-                                              tiles_m, total_tiles, error_flag, grouping.groups,
-                                              columns, clamp);
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = dim3(THREADS);
+    config.dynamicSmemBytes = shared;
+    config.stream = stream;
+    cudaLaunchAttribute cluster[1];
+    cluster[0].id = cudaLaunchAttributeClusterDimension;
+    cluster[0].val.clusterDim.x = 2;
+    cluster[0].val.clusterDim.y = cluster[0].val.clusterDim.z = 1;
+    config.attrs = cluster;
+    config.numAttrs = PAIR ? 1 : 0;
+    cudaLaunchKernelEx(&config, kernel, map_a, map_w, bias, out, ldo, m, n, k, up_offset, tiles_m, total_tiles,
+                       error_flag, grouping.groups, columns, clamp);
     return 0;
 }
 
@@ -534,10 +649,17 @@ MLXONE_API int mlxone_gemm_tcgen05(const void* a, int lda, const void* w, const 
             // SMs: 424 rows of 2 x 6,912 columns of 1,536 are two rounds of either, 24.6 against 28.2
             // us; 528 rows of 2 x 8,192 columns of 2,048 three, 39.4 against 44.5 us. With a round more the
             // operands' additional reads outweigh the smaller tiles (900 rows of the latter, five rounds
-            // against four: 58.6 against 56.5 us).
-            code = gated_rounds(m, n / 2, 96) <= gated_rounds(m, n / 2, 128)
-                       ? launch<192, SWIGLU, MIDDLE_STAGES>(a, lda, w, bias, out, ldo, m, n, k, n / 2, error_flag, stream)
-                       : launch<256, SWIGLU, WIDE_STAGES>(a, lda, w, bias, out, ldo, m, n, k, n / 2, error_flag, stream);
+            // against four: 58.6 against 56.5 us). Otherwise blocks in pairs, unless their larger tiles take
+            // a round more: a block then reads 32 KB for what it read 48 KB for, and these reads are what
+            // bounds a block by itself. Us alone / in pairs, 2,048 rows: 2 x 4,608 columns of 1,024 34.5 / 32.9,
+            // of 2,048 57.5 / 55.0; 2 x 8,192 of 1,024 55.5 / 51.7, of 2,048 100.0 / 94.9 (the library's plain
+            // product 94.6); 4,096 rows of the last 192.4 / 178.8.
+            if (gated_rounds(m, n / 2, 96, 1) <= gated_rounds(m, n / 2, 128, 1))
+                code = launch<192, SWIGLU, MIDDLE_STAGES>(a, lda, w, bias, out, ldo, m, n, k, n / 2, error_flag, stream);
+            else if (gated_rounds(m, n / 2, 128, 2) <= gated_rounds(m, n / 2, 128, 1))
+                code = launch<256, SWIGLU, PAIR_STAGES, true>(a, lda, w, bias, out, ldo, m, n, k, n / 2, error_flag, stream);
+            else
+                code = launch<256, SWIGLU, WIDE_STAGES>(a, lda, w, bias, out, ldo, m, n, k, n / 2, error_flag, stream);
             break;
         case ADD_RESIDUAL:
             code = wide ? launch<256, ADD_RESIDUAL, WIDE_STAGES>(a, lda, w, bias, out, ldo, m, n, k, 0, error_flag, stream)

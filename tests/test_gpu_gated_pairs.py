@@ -1,0 +1,30 @@
+"""The gated tcgen05 product where blocks work in pairs on tiles of 256 rows: full and ragged last tiles, a
+pair whose second block has no rows, rows of the output that 16-byte stores cannot take, one and several
+stages of K, with biases and without."""
+
+import pytest
+import torch
+
+from test_gpu_kernels import ops  # noqa: F401  (fixture)
+
+pytestmark = pytest.mark.gpu
+DEVICE = "cuda:0"
+
+
+@pytest.mark.parametrize("m,width,k", [(1024, 4608, 8), (1000, 4600, 72), (1281, 4605, 64), (1500, 8192, 520),
+                                       (2049, 4608, 136), (1025, 7001, 1032)])
+def test_pairs(ops, m, width, k):
+    rounds = lambda rows, columns, blocks: -(-(-(-m // rows) * -(-width // columns)) // (ops._sm_count // blocks))
+    assert ops._sm_count != 148 or (rounds(128, 96, 1) > rounds(128, 128, 1) >= rounds(256, 128, 2))
+    generator = torch.Generator(DEVICE).manual_seed(m + width + k)
+    a = torch.randn(m, k, generator=generator, device=DEVICE).bfloat16()
+    w = (torch.randn(2 * width, k, generator=generator, device=DEVICE) / k ** 0.5).bfloat16()
+    bias = torch.randn(2 * width, generator=generator, device=DEVICE)
+    for b in (None, bias):
+        got = torch.empty(m, width, dtype=torch.bfloat16, device=DEVICE)
+        ops._tcgen05_call(a, w, b, got, width, ops._SWIGLU)
+        ops.check_errors()
+        gate, up = (a.double() @ w.double().T + (0 if b is None else b.double())).chunk(2, -1)
+        want = gate * torch.sigmoid(gate) * up
+        # the result's rounding to bfloat16, the fast exponential and 32-bit sums of values around one
+        assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4).all()
