@@ -888,9 +888,11 @@ static int prefill_tcgen05(const void* q, const void* kv, const int* block_table
     if (splits == 1) partial = nullptr;
     const int token_tiles = (tokens + tile_tokens - 1) / tile_tokens + requests;     // an upper bound
     const long long all_items = (long long)token_tiles * kv_heads * splits;
-    // tiles of 64 keys and two blocks an SM when there are items for all of those blocks, or
-    // when the items are cut by keys (their parts then run side by side)
-    const bool small_tiles = all_items >= 2LL * g_sm_count || splits > 1;
+    // tiles of 64 keys and two blocks an SM when there are items for all SMs (with 264 items on 148 SMs two
+    // share most of them: 48 launches of a prompt of 16,411 tokens, 16 heads, 141 against 162 us each one
+    // after the other in tiles of 128 keys), or when the items are cut by keys (their parts then run side
+    // by side)
+    const bool small_tiles = all_items >= g_sm_count || splits > 1;
     const int keys = small_tiles ? 64 : 128;
     const int box_keys = page_size < keys ? page_size : keys;
     CUtensorMap map_q, map_kv;
@@ -926,14 +928,9 @@ static int prefill_tcgen05(const void* q, const void* kv, const int* block_table
     const int shared = small_tiles ? Shape<64>::SHARED_BYTES : Shape<128>::SHARED_BYTES;
     // fewer items than SMs (a prompt's portion beside a step's decodes): every block has one
     // item and walks its key tiles one after the other, so two threads share a row's softmax
-    const bool shared_rows = !small_tiles && all_items < g_sm_count;
-    const int threads = ((shared_rows ? 2 : 1) * 4 + 2) * 32;
-    auto kernel = shaped ? (small_tiles ? attention_tcgen05_kernel<64, 1, true>
-                                        : shared_rows ? attention_tcgen05_kernel<128, 2, true>
-                                                      : attention_tcgen05_kernel<128, 1, true>)
-                         : (small_tiles ? attention_tcgen05_kernel<64, 1, false>
-                                        : shared_rows ? attention_tcgen05_kernel<128, 2, false>
-                                                      : attention_tcgen05_kernel<128, 1, false>);
+    const int threads = ((small_tiles ? 1 : 2) * 4 + 2) * 32;
+    auto kernel = shaped ? (small_tiles ? attention_tcgen05_kernel<64, 1, true> : attention_tcgen05_kernel<128, 2, true>)
+                         : (small_tiles ? attention_tcgen05_kernel<64, 1, false> : attention_tcgen05_kernel<128, 2, false>);
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
     if (err != cudaSuccess) {
         mlxone_set_error("attention_prefill_tcgen05: %s", cudaGetErrorString(err));

@@ -15,11 +15,13 @@
 // parts that are none, values near the largest round up to infinity as bfloat16; results below 2^-100)
 // is computed again by one thread in 32-bit FMAs, in the order of gemm_f32.cu.
 //
-// Persistent blocks, one per SM, of 28 warps; tiles of 128 x BN outputs:
+// Persistent blocks, one per SM, of 20 warps; tiles of 128 x BN outputs:
 //   warp 0       one thread issues tcgen05.mma (M = 128, N = BN, K = 16), twelve a section (warps 1-3 idle)
 //   warps 4-11   add up the sections: a quarter of the accumulator's lanes, half of its columns each
-//   warps 12-27  read the operands, 64 values of K a stage, cut them and write the three parts into
-//                shared memory (128-byte swizzle); the next stage's values are under way meanwhile
+//   warps 12-19  read the operands, 64 values of K a stage, cut them and write the three parts into
+//                shared memory (128-byte swizzle); the next stage's values are asked for once a stage is handed
+//                over (asked for between the cuts they made a stage a quarter longer; with 16 warps that
+//                cut it took 4 % longer)
 // Reading each operand tile as it is and cutting it here costs less than a pass that cuts the weights
 // first (134 MB in and 201 MB out for 2048 -> 16384) or keeping three more copies of them.
 #include "common.cuh"
@@ -29,11 +31,11 @@ namespace {
 
 constexpr int BM = 128, BK = 64, SECTION = 32, GROUP = 8;      // GROUP sections: 256 values of K
 constexpr int STAGES = 2, BUFFERS = 2;
-constexpr int SUM_WARPS = 8, CUT_WARPS = 16, FIRST_SUM = 4, FIRST_CUT = FIRST_SUM + SUM_WARPS;
+constexpr int SUM_WARPS = 8, CUT_WARPS = 8, FIRST_SUM = 4, FIRST_CUT = FIRST_SUM + SUM_WARPS;
 constexpr int THREADS = 32 * (FIRST_CUT + CUT_WARPS);
-// registers a thread: 72 at the launch (896 x 72 = 64,512), of which the first four warps and those that
-// cut give up what the ones that add take: 128 x 40 + 256 x 120 + 512 x 56 = 64,512
-constexpr int ISSUE_REGISTERS = 40, SUM_REGISTERS = 120, CUT_REGISTERS = 56;
+// registers a thread: 96 at the launch (640 x 96 = 61,440), of which the first four warps give up what the
+// ones that add take: 128 x 40 + 256 x 120 + 256 x 96 = 60,416
+constexpr int ISSUE_REGISTERS = 40, SUM_REGISTERS = 120, CUT_REGISTERS = 96;
 // results outside of these sizes are computed again in FMAs
 constexpr float LARGEST = 3.0e38f, SMALLEST = 7.9e-31f;
 constexpr int WAIT_LIMIT = 1 << 24;                            // polls before a wait gives up
@@ -439,7 +441,6 @@ gemm_f32_split_kernel(const float* __restrict__ a, int lda, const float* __restr
                     cut(lo[i].z, lo[i].w, h.y, mid.y, l.y);
                     cut(hi[i].x, hi[i].y, h.z, mid.z, l.z);
                     cut(hi[i].z, hi[i].w, h.w, mid.w, l.w);
-                    if (next_tile < total_tiles) fetch(i, next_tile, next_stage);
                     const bool of_a = ROWS * i < BM;
                     const int part = of_a ? A_PART : W_PART;
                     unsigned char* to = base + (of_a ? r * 128 : 3 * A_PART + (r - BM) * 128) +
@@ -451,6 +452,9 @@ gemm_f32_split_kernel(const float* __restrict__ a, int lda, const float* __restr
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) barrier_arrive(full(s));
+                if (next_tile < total_tiles)
+#pragma unroll
+                    for (int i = 0; i < PIECES; ++i) fetch(i, next_tile, next_stage);
             }
         }
         if (BN == 64 && splits > 1) {
