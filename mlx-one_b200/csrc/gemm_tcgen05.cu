@@ -37,7 +37,7 @@ constexpr int EPILOGUE_WARPS = 8, THREADS = 64 + 32 * EPILOGUE_WARPS;  // and a 
 constexpr int WAIT_LIMIT = 1 << 24;    // polls before a wait gives up
 constexpr int ERROR_WAIT = 9;
 
-// (STORE_RELU2: the square of max(z, 0), stored in bfloat16; grouped products only)
+// (STORE_RELU2: the square of max(z, 0), stored in bfloat16)
 enum : int { STORE_BF16 = 0, SWIGLU = 1, ADD_RESIDUAL = 2, STORE_F32 = 3, STORE_RELU2 = 4 };
 __host__ __device__ constexpr bool stores_bf16(int epilogue) {
     return epilogue == STORE_BF16 || epilogue == SWIGLU || epilogue == STORE_RELU2;
@@ -633,7 +633,7 @@ MLXONE_API int mlxone_gemm_tcgen05(const void* a, int lda, const void* w, const 
     MLXONE_REQUIRE((reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
                        (reinterpret_cast<uintptr_t>(w) & 15) == 0,
                    "gemm_tcgen05: operands must be 16-byte aligned");
-    MLXONE_REQUIRE(epilogue >= 0 && epilogue <= 3, "gemm_tcgen05: unknown epilogue %d", epilogue);
+    MLXONE_REQUIRE(epilogue >= 0 && epilogue <= STORE_RELU2, "gemm_tcgen05: unknown epilogue %d", epilogue);
     MLXONE_REQUIRE(epilogue != SWIGLU || n % 2 == 0, "gemm_tcgen05: SwiGLU needs an even n");
     int code;
     // 128 x 256 tiles unless the output is narrower: a 128 x 128 product reads its operands
@@ -660,6 +660,9 @@ MLXONE_API int mlxone_gemm_tcgen05(const void* a, int lda, const void* w, const 
                 code = launch<256, SWIGLU, PAIR_STAGES, true>(a, lda, w, bias, out, ldo, m, n, k, n / 2, error_flag, stream);
             else
                 code = launch<256, SWIGLU, WIDE_STAGES>(a, lda, w, bias, out, ldo, m, n, k, n / 2, error_flag, stream);
+            break;
+        case STORE_RELU2:
+            code = launch<256, STORE_RELU2, PAIR_STAGES, true>(a, lda, w, bias, out, ldo, m, n, k, 0, error_flag, stream);
             break;
         case ADD_RESIDUAL:
             code = wide ? launch<256, ADD_RESIDUAL, WIDE_STAGES>(a, lda, w, bias, out, ldo, m, n, k, 0, error_flag, stream)

@@ -28,3 +28,18 @@ def test_pairs(ops, m, width, k):
         want = gate * torch.sigmoid(gate) * up
         # the result's rounding to bfloat16, the fast exponential and 32-bit sums of values around one
         assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(1024, 4096, 8), (1000, 4090, 72), (1281, 8192, 64), (2049, 4100, 136),
+                                   (1500, 8191, 1032)])
+def test_squared_relu(ops, m, n, k):
+    generator = torch.Generator(DEVICE).manual_seed(m + n + k)
+    a = torch.randn(m, k, generator=generator, device=DEVICE).bfloat16()
+    w = (torch.randn(n, k, generator=generator, device=DEVICE) / k ** 0.5).bfloat16()
+    got = torch.empty(m, n, dtype=torch.bfloat16, device=DEVICE)
+    ops._tcgen05_call(a, w, None, got, n, ops._RELU2)
+    ops.check_errors()
+    want = torch.relu(a.double() @ w.double().T) ** 2
+    # the result's rounding to bfloat16, and 32-bit sums of values around one, squared
+    assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4).all()
+    assert torch.equal(ops.linear_act(a, w, "relu2"), got) or not ops._tcgen05(a, w, ops._RELU2)
