@@ -575,6 +575,23 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv,
     }
     griddep_wait();
     for (; ahead < DECODE_STAGES - 1; ++ahead) fetch(ahead);
+    // The token's own key and value (the warp that will meet their tile), asked for beside the queries and
+    // not behind them. Lane e takes dims e, e + 32, ...: a rotation pair (j, j + HD / 2) lies in one lane.
+    float k_lo[KEY_PAIRS], k_hi[KEY_PAIRS], v_lo[KEY_PAIRS], v_hi[KEY_PAIRS];
+    if (PREP && meets_newest) {
+        const bf16* row = q + (size_t)request * (heads + 2 * kv_heads) * HD;
+        const bf16* k_src = row + (size_t)(heads + kv_head) * HD;
+        const bf16* v_src = row + (size_t)(heads + kv_heads + kv_head) * HD;
+#pragma unroll
+        for (int i = 0; i < KEY_PAIRS; ++i) {
+            const int j = lane + 32 * i;
+            const bool mine = j < HD / 2;
+            k_lo[i] = mine ? __bfloat162float(k_src[j]) : 0.f;
+            k_hi[i] = mine ? __bfloat162float(k_src[j + HD / 2]) : 0.f;
+            v_lo[i] = mine ? __bfloat162float(v_src[j]) : 0.f;
+            v_hi[i] = mine ? __bfloat162float(v_src[j + HD / 2]) : 0.f;
+        }
+    }
 
     // q^T as the 8-column operand: head g, dims 16 kk + 2t (+1) and + 8
     uint32_t qb[HD / 16][2];
@@ -628,26 +645,11 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv,
             }
         }
     }
-    // The token's own key and value (the warp that will meet their tile): normed and rotated
-    // here from the projection's row, while the first tiles are on their way. Lane e takes dims
-    // e, e + 32, ...: a rotation pair (j, j + HD / 2) lies in one lane.
-    float k_lo[KEY_PAIRS], k_hi[KEY_PAIRS], v_lo[KEY_PAIRS], v_hi[KEY_PAIRS];
+    // the token's own key, normed and rotated while the first tiles are on their way
     if (PREP && meets_newest) {
-        constexpr int HALF = HD / 2;
-        const bf16* row = q + (size_t)request * (heads + 2 * kv_heads) * HD;
-        const bf16* k_src = row + (size_t)(heads + kv_head) * HD;
-        const bf16* v_src = row + (size_t)(heads + kv_heads + kv_head) * HD;
         float sum = 0.f;
 #pragma unroll
-        for (int i = 0; i < KEY_PAIRS; ++i) {
-            const int j = lane + 32 * i;
-            const bool mine = j < HALF;
-            k_lo[i] = mine ? __bfloat162float(k_src[j]) : 0.f;
-            k_hi[i] = mine ? __bfloat162float(k_src[j + HALF]) : 0.f;
-            v_lo[i] = mine ? __bfloat162float(v_src[j]) : 0.f;
-            v_hi[i] = mine ? __bfloat162float(v_src[j + HALF]) : 0.f;
-            sum += k_lo[i] * k_lo[i] + k_hi[i] * k_hi[i];
-        }
+        for (int i = 0; i < KEY_PAIRS; ++i) sum += k_lo[i] * k_lo[i] + k_hi[i] * k_hi[i];
         if (prep.k_weight != nullptr) {
             sum = warp_sum(sum);
             const float inv = rsqrtf(sum / (float)HD + prep.eps);
