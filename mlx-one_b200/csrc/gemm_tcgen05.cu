@@ -300,6 +300,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                                     up_offset + tile_n, full(s));
                 }
             }
+            // The last stages' products report here too (in pairs the first block's commits write into this
+            // block's memory): nothing else waits for them, and a block must not be gone when they land.
+            for (int last = max(0, step - STAGES); last < step && ok; ++last)
+                ok = barrier_wait(empty(last % STAGES), (last / STAGES) & 1, error_flag);
         }
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {

@@ -43,3 +43,20 @@ def test_squared_relu(ops, m, n, k):
     # the result's rounding to bfloat16, and 32-bit sums of values around one, squared
     assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4).all()
     assert torch.equal(ops.linear_act(a, w, "relu2"), got) or not ops._tcgen05(a, w, ops._RELU2)
+
+
+@pytest.mark.parametrize("k", [64, 320, 384, 448])         # fewer stages of K than the ring has, as many, more
+def test_pairs_one_after_the_other(ops, k):
+    """A block leaves once its last stages' products have reported, so that the blocks which take its place
+    find their barriers untouched: products without a pause between them have the bits of the first."""
+    generator = torch.Generator(DEVICE).manual_seed(k)
+    a = torch.randn(1281, k, generator=generator, device=DEVICE).bfloat16()
+    w = (torch.randn(2 * 4608, k, generator=generator, device=DEVICE) / k ** 0.5).bfloat16()
+    gated = [torch.empty(1281, 4608, dtype=torch.bfloat16, device=DEVICE) for _ in range(40)]
+    squared = [torch.empty(1281, 2 * 4608, dtype=torch.bfloat16, device=DEVICE) for _ in range(40)]
+    for one, other in zip(gated, squared):
+        ops._tcgen05_call(a, w, None, one, 4608, ops._SWIGLU)
+        ops._tcgen05_call(a, w, None, other, 2 * 4608, ops._RELU2)
+    ops.check_errors()
+    assert all(torch.equal(gated[0], one) for one in gated)
+    assert all(torch.equal(squared[0], one) for one in squared)
