@@ -464,6 +464,9 @@ gemm_f32_split_kernel(const float* __restrict__ a, int lda, const float* __restr
                     for (int i = 0; i < PIECES; ++i) fetch(i, next_tile, next_stage);
             }
         }
+        // (the last stages' products report to nobody else, and a block must not be gone when they do)
+        for (int last = max(0, step - STAGES); last < step && ok; ++last)
+            ok = barrier_wait(empty(last % STAGES), (last / STAGES) & 1, error_flag);
         if (BN == 64 && splits > 1) {
             __syncwarp();
             cluster_barrier();
