@@ -574,12 +574,13 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv,
         }
     }
     griddep_wait();
+    const bf16* written = settled(q);          // (what the kernel before this one wrote)
     for (; ahead < DECODE_STAGES - 1; ++ahead) fetch(ahead);
     // The token's own key and value (the warp that will meet their tile), asked for beside the queries and
     // not behind them. Lane e takes dims e, e + 32, ...: a rotation pair (j, j + HD / 2) lies in one lane.
     float k_lo[KEY_PAIRS], k_hi[KEY_PAIRS], v_lo[KEY_PAIRS], v_hi[KEY_PAIRS];
     if (PREP && meets_newest) {
-        const bf16* row = q + (size_t)request * (heads + 2 * kv_heads) * HD;
+        const bf16* row = written + (size_t)request * (heads + 2 * kv_heads) * HD;
         const bf16* k_src = row + (size_t)(heads + kv_head) * HD;
         const bf16* v_src = row + (size_t)(heads + kv_heads + kv_head) * HD;
 #pragma unroll
@@ -598,7 +599,7 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv,
     {
         const bool live = g < rows;
         const size_t row_stride = PREP ? (size_t)(heads + 2 * kv_heads) * HD : (size_t)heads * HD;
-        const bf16* row = q + (size_t)request * row_stride + (size_t)(head0 + (live ? g : 0)) * HD;
+        const bf16* row = written + (size_t)request * row_stride + (size_t)(head0 + (live ? g : 0)) * HD;
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
             qb[kk][0] = live ? *reinterpret_cast<const uint32_t*>(row + kk * 16 + 2 * t) : 0u;

@@ -86,3 +86,36 @@ def test_same_logits_in_32_bit_and_with_the_delta_rule(tmp_path, name, dtype):
     finally:
         ops.set_dependent_launches(True)
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(32, 8, 64), (16, 8, 64), (8, 2, 128)])
+def test_decode_attention_reads_its_row_behind_the_wait(heads, kv_heads, head_dim):
+    """A projection and the decode attention that starts from its row, two inputs in turn through one buffer:
+    a query, key or value asked for ahead of the wait would be the other input's."""
+    from mlx_one_b200.kernels.cuda_ops import CudaOps
+    from mlx_one_b200.parts.base import PagedKeyValues, PagedView
+    from test_gpu_kernels import make_batch
+
+    ops, hidden = CudaOps("cuda:0", verbose=False), 4096
+    generator = torch.Generator("cuda:0").manual_seed(head_dim)
+    normal = lambda *shape: torch.randn(shape, generator=generator, device="cuda:0").bfloat16()
+    w, inputs = normal((heads + 2 * kv_heads) * head_dim, hidden) / 64, [normal(4, hidden) for _ in range(2)]
+    ctx, table, pages = make_batch([1] * 4, [0, 31, 70, 700], 16, "cuda:0")
+    kv = normal(2, pages, kv_heads, 16, head_dim)
+    need = PagedKeyValues(kv_heads, head_dim, None)
+    results = []
+    try:
+        for enabled in (False, True):
+            ops.set_dependent_launches(enabled)
+            for i in range(400):
+                qkv = ops.linear(inputs[i % 2], w)
+                got = ops.qkv_attention(qkv, q_weight=None, k_weight=None, rotary=None, ctx=ctx, eps=None,
+                                        view=PagedView(kv, table, 16, need), heads=heads, kv_heads=kv_heads,
+                                        head_dim=head_dim, scale=0.125, window=None, write=True)
+                del qkv
+                results.append(got)
+    finally:
+        ops.set_dependent_launches(True)
+    ops.check_errors()
+    assert not torch.equal(results[0], results[1])
+    assert all(torch.equal(got, results[i % 2]) for i, got in enumerate(results))
