@@ -3,7 +3,8 @@
 // Plain FMA on CUDA cores, no tensor cores and no reduced-precision mode. A row's result does not
 // depend on how many other rows the call has, on where its tile lies or on which of the kernels
 // below computed it: every output is added up in the same order, a function of K alone. (Products of more
-// than 130 rows that 16-byte loads can take are gemm_f32_tcgen05.cu's, in another order.)
+// than 130 rows that 16-byte loads can take are gemm_f32_tcgen05.cu's, whose order is a function of K alone too,
+// but another: a row's last bits are not the same on both sides of that line.)
 //
 //   strand   one chain of up to 32 FMAs from zero: of a section of 256 values of K, strand l takes
 //            the pieces of eight values at 64 j + 8 l, j = 0 .. 3, in ascending order

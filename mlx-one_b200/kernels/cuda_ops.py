@@ -6,8 +6,8 @@ pointers and the current CUDA stream to the library. There is no fallback: const
 
 Matrix products in bfloat16 go through ``torch.matmul`` (cuBLAS), as the reference uses its
 library's matrix product (nn.Linear, src/mlx_one/models/language/lfm2/reference_math.py:33-34);
-in float32 they go through this library's own FMA kernel, which never uses a
-reduced-precision mode.
+in float32 they go through this library's own kernels: FMAs, and for many rows eight bfloat16
+products of the values' parts (24 bits of every value, sums in 32 bits).
 """
 
 from __future__ import annotations
@@ -76,7 +76,12 @@ class CudaOps:
         self.fused_norms = True
         self.fused_norm_max_rows = 6
         # 32-bit products of more rows than this on the tensor cores, each value cut into three bfloat16
-        # parts (csrc/gemm_f32_tcgen05.cu). Up to here all kernels add a row up in the same order.
+        # parts (csrc/gemm_f32_tcgen05.cu). Both sides of the line have one order of additions, a function of K
+        # alone, but not the same one. 128 rows are a tile of the FMA kernels, a second one begins behind them:
+        # us on the tensor cores / by FMAs at 128 and 131 rows: 2048 -> 16384 93 / 220 and 182 / 357, 8192 -> 2048
+        # 88 / 158 and 163 / 277, 2048 -> 6144 86 / 119 and 89 / 138, 1024 -> 1024 20 / 25 and 20 / 24; 2048 -> 3072 52 / 71 but
+        # 84 / 71 (up to 160 rows; 85 / 113 at 200). Faster below the line as well, from 64 rows on in most; there the FMA
+        # kernels' bits hold, which a step of up to 130 rows shares with single tokens.
         self.f32_split = True
         self.f32_split_rows = 130
         self.tcgen05_min_rows = 128
