@@ -29,7 +29,8 @@
 //
 // An output that does not come out as an ordinary number (infinities and NaN in the inputs, inputs of 2^112 and
 // more and results of 2^95 and more, which the scale takes out of range; results below 2^-132) is computed again
-// by one thread in 32-bit FMAs, in the order of gemm_f32.cu.
+// by a warp in 32-bit FMAs, in the order of gemm_f32.cu. That is slow: 2048 -> 16384 at 1,200 rows takes 803 us, 1,230
+// with one infinity among the inputs (a row of outputs), 2,550 with 19 rows of 2^115, 85 ms where all results are tiny.
 //
 // Persistent blocks, one per SM, of 20 warps; tiles of 128 x BN outputs:
 //   warp 0       one thread issues tcgen05.mma (M = 128, K = 16): the leading products, then, while those are
@@ -180,22 +181,22 @@ __device__ __forceinline__ bool needs_plain(float value) {
     return !(size <= LARGEST) || (size < SMALLEST && size > 0.f);
 }
 
-// One output as gemm_f32.cu adds it up (strands of 32 values, sections of 256). Not inlined: it is
-// all but never called.
+// One output as gemm_f32.cu adds it up (strands of 32 values, sections of 256), by a warp: a strand a
+// lane, four sections at a time. Not inlined: it is all but never called.
 __device__ __noinline__ float plain_product(const float* a, const float* w, int k) {
+    const int lane = threadIdx.x & 31;
     float total = 0.f;
-    for (int section = 0; section < k; section += 256) {
-        float sum = 0.f;
-        for (int strand = 0; strand < 8; ++strand) {
-            float acc = 0.f;
-            for (int j = 0; j < 4; ++j) {
-                const int at = section + 64 * j + 8 * strand;
-                if (at < k)                                     // (K is a multiple of 8)
-                    for (int i = 0; i < 8; ++i) acc = fmaf(a[at + i], w[at + i], acc);
-            }
-            sum += acc;
+    for (int first = 0; first < k; first += 4 * GROUP) {
+        float strand = 0.f;
+        for (int j = 0; j < 4; ++j) {
+            const int at = first + (lane >> 3) * GROUP + 64 * j + 8 * (lane & 7);
+            if (at < k)                                         // (K is a multiple of 8)
+                for (int i = 0; i < 8; ++i) strand = fmaf(a[at + i], w[at + i], strand);
         }
-        total += sum;
+        float section = 0.f;
+        for (int i = 0; i < 8; ++i) section += __shfl_sync(0xffffffffu, strand, i, 8);
+        for (int i = 0; i < 4; ++i)
+            if (first + i * GROUP < k) total += __shfl_sync(0xffffffffu, section, 8 * i);
         if (total != total) break;                              // NaN stays
     }
     return total;
@@ -448,10 +449,13 @@ gemm_f32_split_kernel(const float* __restrict__ a, int lda, const float* __restr
             }
 #pragma unroll
             for (int c = 0; c < COLUMNS; c += 16)
-                for (uint32_t left = again[c / 16]; left != 0; left &= left - 1) {
-                    const int column = column0 + c + __ffs(left) - 1;
-                    const float value = plain_product(a + (size_t)row * lda, w + (size_t)column * ldw, k);
-                    out[(size_t)row * ldo + column] = value + (bias != nullptr ? bias[column] : 0.f);
+                for (uint32_t those = __ballot_sync(0xffffffffu, again[c / 16] != 0); those != 0; those &= those - 1) {
+                    const int whose = __ffs(those) - 1, its_row = row - lane + whose;
+                    for (uint32_t left = __shfl_sync(0xffffffffu, again[c / 16], whose); left != 0; left &= left - 1) {
+                        const int column = column0 + c + __ffs(left) - 1;
+                        const float value = plain_product(a + (size_t)its_row * lda, w + (size_t)column * ldw, k);
+                        if (lane == whose) out[(size_t)row * ldo + column] = value + (bias != nullptr ? bias[column] : 0.f);
+                    }
                 }
             __syncwarp();
         }
@@ -483,7 +487,13 @@ gemm_f32_split_kernel(const float* __restrict__ a, int lda, const float* __restr
                 for (int j = 0; j < 4; ++j) {
                     const bool again = needs_plain(value[j]) && row < m && column + j < n;
                     value[j] *= UNSCALE;
-                    if (again) value[j] = plain_product(a + (size_t)row * lda, w + (size_t)(column + j) * ldw, k);
+                    for (uint32_t those = __ballot_sync(0xffffffffu, again); those != 0; those &= those - 1) {
+                        const int whose = __ffs(those) - 1;
+                        const float plain =
+                            plain_product(a + (size_t)__shfl_sync(0xffffffffu, row, whose) * lda,
+                                          w + (size_t)__shfl_sync(0xffffffffu, column + j, whose) * ldw, k);
+                        if (lane == whose) value[j] = plain;
+                    }
                     if (bias != nullptr && column + j < n) value[j] += bias[column + j];
                 }
                 if (row >= m) continue;

@@ -162,3 +162,26 @@ def test_values_beyond_the_scale(ops, m, n, k):
     want, allowed = a.double() @ w.double().T, bound(a, w)
     for row in (0, 7, 9):
         assert ((got[row].double() - want[row]).abs() <= allowed[row] + 2.0 ** -149).all(), row
+
+
+def test_an_infinity_costs_little(ops):
+    """The outputs of a row with an infinity are computed again by FMAs, a warp each (by a thread each the call took
+    fifteen times as long, now one and a half)."""
+    generator = torch.Generator(DEVICE).manual_seed(5)
+    a, w = (torch.randn(rows, 2048, generator=generator, device=DEVICE) for rows in (1200, 16384))
+    odd = a.clone()
+    odd[17, 3] = float("inf")
+
+    def milliseconds(x):
+        times = []
+        for _ in range(4):
+            events = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            events[0].record()
+            ops.linear(x, w)
+            events[1].record()
+            torch.cuda.synchronize()
+            times.append(events[0].elapsed_time(events[1]))
+        return min(times)
+
+    assert milliseconds(odd) < 6 * milliseconds(a)
+    ops.check_errors()
