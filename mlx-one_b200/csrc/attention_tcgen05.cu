@@ -49,11 +49,11 @@ constexpr int HD = 64;
 constexpr int ROWS = 128;              // query rows per block
 constexpr int STAGES = 3;              // ring of key/value tiles
 // PARTS (a parameter of the kernel): threads that share a query row, each for its share of a
-// tile's keys and of the output dimensions. One: a thread owns its row's scores of a tile and
-// all of its output, and the softmax warps exchange nothing, which is the faster form when an SM
-// has several items to overlap (8192 tokens: 603 against 556 TFLOP/s). Two: a tile's softmax
-// takes half as long, which is what counts when a block has one item and nothing beside it, the
-// portion of a prompt in a step of decodes (see the launch).
+// tile's keys and of the output dimensions. One (tiles of 64 keys): a thread owns its row's scores of a
+// tile and all of its output, and the softmax warps exchange nothing, which is the faster form when an SM
+// has several items to overlap (8192 tokens: 603 against 556 TFLOP/s). Two (tiles of 128 keys): a tile's
+// softmax takes half as long, which is what counts when an SM has one block (one or two items of it, 144 to 288
+// of a prompt: 2 to 7 % faster than one thread a row where contexts are short, as fast where they are long).
 constexpr int WAIT_LIMIT = 1 << 24;
 constexpr int ERROR_WAIT = 9;
 constexpr int Q_BYTES = ROWS * HD * 2;
@@ -61,7 +61,8 @@ constexpr int Q_BYTES = ROWS * HD * 2;
 // Two shapes of the kernel. With 128 keys a tile a block fills an SM (tensor memory: scores
 // 2 x 128 columns, output 64); with 64 keys a tile two blocks share an SM, and while one waits
 // for a product or a barrier the other computes: faster when there are items for all of them,
-// slower when there are not, since a block then walks its keys in more, smaller steps.
+// slower when there are not, since a block then walks its keys in more, smaller steps
+// (mlxone_attention_tcgen05_keys draws the line).
 template <int KEYS_>
 struct Shape {
     static constexpr int KEYS = KEYS_;
@@ -794,6 +795,16 @@ typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, v
 EncodeTiled g_encode = nullptr;
 int g_sm_count = 0;
 
+int sm_count() {
+    if (g_sm_count == 0) {
+        int device = 0;
+        cudaGetDevice(&device);
+        cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, device);
+        if (g_sm_count <= 0) g_sm_count = 148;
+    }
+    return g_sm_count;
+}
+
 bool find_encoder() {
     if (g_encode != nullptr) return true;
     void* fn = nullptr;
@@ -831,21 +842,46 @@ MLXONE_API int mlxone_attention_tcgen05_supports(int head_dim, int heads, int kv
 MLXONE_API int mlxone_attention_tcgen05_splits(int tokens, int requests, int heads, int kv_heads,
                                                int max_context) {
     if (tokens <= 0 || requests <= 0 || kv_heads <= 0 || heads % kv_heads != 0) return 1;
-    if (g_sm_count == 0) {
-        int device = 0;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, device);
-        if (g_sm_count <= 0) g_sm_count = 148;
-    }
     const int tile_tokens = ROWS / (heads / kv_heads);
     if (tile_tokens < 1) return 1;
     const long long items = (long long)((tokens + tile_tokens - 1) / tile_tokens + requests) * kv_heads;
-    if (items >= g_sm_count) return 1;
-    long long splits = 2LL * g_sm_count / items;
+    if (items >= sm_count()) return 1;
+    long long splits = 2LL * sm_count() / items;
     const long long by_keys = max_context / 64 / 6;
     if (splits > by_keys) splits = by_keys;
     if (splits > 8) splits = 8;
     return splits < 1 ? 1 : (int)splits;
+}
+
+// Keys a tile: 64 (two blocks an SM) or 128 (one, two threads a query row). Items (128 query rows of a key head)
+// are estimated, since portions end amid tiles: half a tile more for every request but one.
+//   cut by keys, or two items for every SM: 64.
+//   fewer items than SMs: 128, as every block walks one item (144 items, 8,192 earlier keys: 131 against 155 us).
+//   between, several requests: 64. (2 to 8 requests of 190 to 288 items: 1.1 to 1.4 times as fast, of fewer 0.9 to 1.2;
+//   15 % slower where one request of four has most of the keys.)
+//   between, one request: the launch lasts as long as its longest item. A causal prompt's heavy and light items
+//   pair off in one block of an SM: 128, until the earlier keys make all items alike. Us in tiles of 64 / 128 keys, 16
+//   heads over 8, 2,048 tokens behind 0 / 2,048 / 4,096 / 8,192 keys: 35.2 / 27.5, 65.0 / 64.6, 95.3 / 103.6, 154.6 / 180.0;
+//   32 heads, 704 tokens behind 0 / 512 / 2,048 / 8,192: 16.5 / 14.4, 24.0 / 22.5, 45.9 / 50.3, 135 / 165. So from one and a
+//   half times the portion's length on 64 (within 7 % of the better one on both sides), but not with a ragged last
+//   tile, whose rows are masked throughout: beside another block that one takes longest (2,016 tokens behind 8,192:
+//   198 / 180). A window that earlier keys fill, or that the portion passes twice, makes items alike and short (1,019
+//   tokens of 32 heads behind 6,000 keys: window of 512 20.8 / 24.6, 1,024 31.0 / 33.3, 4,096 91.7 / 89.8; 1,339 tokens of
+//   24 heads behind none, window of 512 19.0 / 23.0). Scores with a cap or a bias: the same lines (1,051 tokens of 32
+//   heads behind none 34.6 / 29.3, 1,056 behind 8,192 216 / 245).
+MLXONE_API int mlxone_attention_tcgen05_keys(int tokens, int requests, int heads, int kv_heads, int max_context,
+                                             int window, int splits) {
+    if (splits > 1 || tokens <= 0 || kv_heads <= 0 || heads < kv_heads) return 64;
+    const int tile_tokens = ROWS / (heads / kv_heads);
+    if (tile_tokens < 1) return 64;
+    const long long twice = (2LL * ((tokens + tile_tokens - 1) / tile_tokens) + requests - 1) * kv_heads;
+    const int sms = sm_count();
+    if (twice >= 4LL * sms) return 64;
+    if (twice < 2LL * sms) return 128;
+    if (requests > 1) return 64;
+    const int earlier = max_context - tokens, span = window < 0 ? -window : window;
+    if (span > 0 && span <= 4096 && (earlier >= span || tokens >= 2LL * span)) return 64;
+    return tokens % tile_tokens == 0 && 2LL * earlier >= 3LL * tokens ? 64 : 128;
 }
 
 // q: [tokens, heads, 64] bfloat16; kv: [2, pages, kv_heads, page_size, 64]; out: [tokens, heads * 64].
@@ -858,7 +894,7 @@ static int prefill_tcgen05(const void* q, const void* kv, const int* block_table
                                                 void* out, int tokens, int requests, int heads,
                                                 int kv_heads, int head_dim, float scale, int window,
                                                 int splits, float* partial, const float* sinks,
-                                                int* error_flag, cudaStream_t stream, int keep_first,
+                                                int keys, int* error_flag, cudaStream_t stream, int keep_first,
                                                 bool shaped = false, ScoreShape shape = ScoreShape()) {
     if (tokens == 0) return 0;
     MLXONE_REQUIRE(keep_first >= 0 && (keep_first == 0 || window > 0),
@@ -877,23 +913,14 @@ static int prefill_tcgen05(const void* q, const void* kv, const int* block_table
     const int tile_tokens = ROWS / group;
     const long long value_rows = (long long)pages * kv_heads * page_size;
     MLXONE_REQUIRE(2 * value_rows < (1LL << 31), "attention_prefill_tcgen05: the cache has too many rows");
-    if (g_sm_count == 0) {
-        int device = 0;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, device);
-        if (g_sm_count <= 0) g_sm_count = 148;
-    }
     MLXONE_REQUIRE(splits >= 1 && splits <= 64 && (splits == 1 || partial != nullptr),
                    "attention_prefill_tcgen05: %d splits need a scratch buffer", splits);
     if (splits == 1) partial = nullptr;
     const int token_tiles = (tokens + tile_tokens - 1) / tile_tokens + requests;     // an upper bound
     const long long all_items = (long long)token_tiles * kv_heads * splits;
-    // tiles of 64 keys and two blocks an SM when there are items for all SMs (with 264 items on 148 SMs two
-    // share most of them: 48 launches of a prompt of 16,411 tokens, 16 heads, 141 against 162 us each one
-    // after the other in tiles of 128 keys), or when the items are cut by keys (their parts then run side
-    // by side)
-    const bool small_tiles = all_items >= g_sm_count || splits > 1;
-    const int keys = small_tiles ? 64 : 128;
+    MLXONE_REQUIRE(keys == 64 || (keys == 128 && splits == 1),
+                   "attention_prefill_tcgen05: tiles of %d keys with %d splits", keys, splits);
+    const bool small_tiles = keys == 64;
     const int box_keys = page_size < keys ? page_size : keys;
     CUtensorMap map_q, map_kv;
     {
@@ -922,12 +949,10 @@ static int prefill_tcgen05(const void* q, const void* kv, const int* block_table
     }
     // persistent blocks, as many as the GPU holds at once; more only if a block would get more
     // items than it can list
-    const long long resident = (long long)g_sm_count * (small_tiles ? 2 : 1);
+    const long long resident = (long long)sm_count() * (small_tiles ? 2 : 1);
     long long blocks = all_items < resident ? all_items : resident;
     if ((all_items + blocks - 1) / blocks > MAX_ITEMS) blocks = (all_items + MAX_ITEMS - 1) / MAX_ITEMS;
     const int shared = small_tiles ? Shape<64>::SHARED_BYTES : Shape<128>::SHARED_BYTES;
-    // fewer items than SMs (a prompt's portion beside a step's decodes): every block has one
-    // item and walks its key tiles one after the other, so two threads share a row's softmax
     const int threads = ((small_tiles ? 1 : 2) * 4 + 2) * 32;
     auto kernel = shaped ? (small_tiles ? attention_tcgen05_kernel<64, 1, true> : attention_tcgen05_kernel<128, 2, true>)
                          : (small_tiles ? attention_tcgen05_kernel<64, 1, false> : attention_tcgen05_kernel<128, 2, false>);
@@ -950,10 +975,10 @@ MLXONE_API int mlxone_attention_prefill_tcgen05(const void* q, const void* kv, c
                                                 void* out, int tokens, int requests, int heads,
                                                 int kv_heads, int head_dim, float scale, int window,
                                                 int splits, float* partial, const float* sinks,
-                                                int* error_flag, cudaStream_t stream) {
+                                                int keys, int* error_flag, cudaStream_t stream) {
     return prefill_tcgen05(q, kv, block_table, table_width, page_size, pages, request_start, history,
                            out, tokens, requests, heads, kv_heads, head_dim, scale, window, splits,
-                           partial, sinks, error_flag, stream, 0);
+                           partial, sinks, keys, error_flag, stream, 0);
 }
 
 // ... with a window behind which the first `keep_first` positions of a sequence stay visible
@@ -964,11 +989,11 @@ MLXONE_API int mlxone_attention_prefill_tcgen05_keep(const void* q, const void* 
                                                      void* out, int tokens, int requests, int heads,
                                                      int kv_heads, int head_dim, float scale,
                                                      int window, int keep_first, int splits,
-                                                     float* partial, const float* sinks,
+                                                     float* partial, const float* sinks, int keys,
                                                      int* error_flag, cudaStream_t stream) {
     return prefill_tcgen05(q, kv, block_table, table_width, page_size, pages, request_start, history,
                            out, tokens, requests, heads, kv_heads, head_dim, scale, window, splits,
-                           partial, sinks, error_flag, stream, keep_first);
+                           partial, sinks, keys, error_flag, stream, keep_first);
 }
 
 // ... with scores s that become cap tanh(s / cap) (cap 0: none) and then lose slopes[head] (float32
@@ -980,9 +1005,9 @@ MLXONE_API int mlxone_attention_prefill_tcgen05_shaped(const void* q, const void
                                                        void* out, int tokens, int requests, int heads,
                                                        int kv_heads, int head_dim, float scale,
                                                        float cap, const float* slopes, int splits,
-                                                       float* partial, int* error_flag,
+                                                       float* partial, int keys, int* error_flag,
                                                        cudaStream_t stream) {
     return prefill_tcgen05(q, kv, block_table, table_width, page_size, pages, request_start, history,
                            out, tokens, requests, heads, kv_heads, head_dim, scale, 0, splits, partial,
-                           nullptr, error_flag, stream, 0, true, make_score_shape(scale, cap, slopes));
+                           nullptr, keys, error_flag, stream, 0, true, make_score_shape(scale, cap, slopes));
 }

@@ -1720,6 +1720,9 @@ class CudaOps:
                     splits = self.lib.mlxone_attention_tcgen05_splits(
                         _c_int(tokens - singles), _c_int(rest), _c_int(heads), _c_int(kv_heads),
                         _c_int(bound))
+                keys = self.lib.mlxone_attention_tcgen05_keys(
+                    _c_int(tokens - singles), _c_int(rest), _c_int(heads), _c_int(kv_heads),
+                    _c_int(ctx.max_context), _c_int(window or 0), _c_int(splits))
                 partial = None
                 if splits > 1:
                     partial = torch.empty(tokens * heads * splits * (head_dim + 2),
@@ -1731,7 +1734,7 @@ class CudaOps:
                            _c_void_p(_ptr(out)), _c_int(tokens), _c_int(rest),
                            _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_float(scale),
                            _c_int(window or 0), _c_int(keep_first), _c_int(splits),
-                           _c_void_p(_ptr(partial)), _c_void_p(_ptr(sinks)),
+                           _c_void_p(_ptr(partial)), _c_void_p(_ptr(sinks)), _c_int(keys),
                            _c_void_p(_ptr(self.error_flag)))
                 if partial is not None:
                     # (the leading single tokens are the decode kernel's: their rows stay)
@@ -1864,8 +1867,11 @@ class CudaOps:
         if splits > 1:
             partial = torch.empty(tokens * heads * splits * (head_dim + 2), dtype=torch.float32,
                                   device=self.device)
+        keys = self.lib.mlxone_attention_tcgen05_keys(
+            _c_int(tokens - singles), _c_int(rest), _c_int(heads), _c_int(kv_heads), _c_int(ctx.max_context),
+            _c_int(reach or 0), _c_int(splits))
         self._call("mlxone_attention_prefill_tcgen05_shaped", *common, _c_int(splits),
-                   _c_void_p(_ptr(partial)), _c_void_p(_ptr(self.error_flag)))
+                   _c_void_p(_ptr(partial)), _c_int(keys), _c_void_p(_ptr(self.error_flag)))
         if partial is not None:
             skip = singles * heads * splits * (head_dim + 2)
             self._call("mlxone_attention_merge", _c_void_p(_ptr(partial[skip:])),

@@ -1,5 +1,5 @@
-"""Prefill attention with one to two items an SM (tiles of 64 keys, two blocks an SM), the gate kernel's
-16-byte pieces and its single values, and how many parts decode attention cuts few keys into."""
+"""Prefill attention with one to two items an SM (tiles of 128 keys, or of 64 with two blocks an SM), the gate
+kernel's 16-byte pieces and its single values, and how many parts decode attention cuts few keys into."""
 
 import pytest
 import torch
@@ -40,3 +40,29 @@ def test_parts_of_few_keys(ops):
         blocks = resident // wanted
         assert ops.decode_splits(blocks, 1, 1, 64, 1024, None) == parts
         assert ops.decode_splits(blocks, 1, 1, 64, 2048, None) == wanted
+
+
+@pytest.mark.parametrize("tokens,requests,heads,max_context,window,keys", [
+    (704, 1, 32, 704, 0, 128), (704, 1, 32, 1216, 0, 128), (704, 1, 32, 2752, 0, 64), (688, 1, 32, 2752, 0, 128),
+    (2048, 1, 16, 2048, 0, 128), (2048, 1, 16, 4096, 0, 128), (2048, 1, 16, 6144, 0, 64), (2016, 1, 16, 8192, 0, 128),
+    (735, 1, 24, 9000, 0, 128),                     # 144 items: fewer than SMs
+    (560, 1, 32, 9000, 0, 128), (2304, 1, 16, 2304, 0, 128), (2368, 1, 16, 2368, 0, 64),    # ... two for every SM
+    (1019, 1, 32, 7019, 1024, 64), (1019, 1, 32, 1019, 1024, 128), (1043, 1, 32, 1043, 512, 64),
+    (1019, 1, 32, 7019, -512, 64),
+    (512, 4, 32, 200, 0, 128), (608, 4, 32, 152, 0, 64), (320, 16, 32, 20, 0, 128), (256, 64, 32, 4, 0, 64)])
+def test_keys_a_tile(ops, tokens, requests, heads, max_context, window, keys):
+    """At the measured points on both sides of every line."""
+    if ops._sm_count != 148:
+        pytest.skip("the lines lie where 148 SMs put them")
+    assert ops.lib.mlxone_attention_tcgen05_keys(tokens, requests, heads, 8, max_context, window, 1) == keys
+    assert ops.lib.mlxone_attention_tcgen05_keys(tokens, requests, heads, 8, max_context, window, 2) == 64
+
+
+@pytest.mark.parametrize("portions,histories,window", [
+    ([1216], [2500], None), ([1216], [100], None), ([1190], [2500], None), ([1184], [1500], 512), ([1190], [40], 300),
+    ([592, 592], [40, 700], None)])
+def test_prefill_on_both_sides_of_the_line(ops, plain, portions, histories, window):
+    """152 items of 16 heads over 8: one request, whole and ragged last tiles behind few and many keys and with
+    windows; two requests."""
+    attention_case(ops, plain, torch.bfloat16, 16, 8, 64, 16, portions=portions, histories=histories,
+                   window=window, tensor_cores=True, tcgen05=True)
