@@ -270,9 +270,9 @@ class CudaOps:
         return picked, picked_delta
 
     # epilogues of the skinny product
-    _STORE, _SWIGLU, _ADD, _STORE_F32, _RELU2 = 0, 1, 2, 3, 4
+    _STORE, _SWIGLU, _ADD, _STORE_F32 = 0, 1, 2, 3
     _ACTIVATE = 16          # + the activation's code: a bfloat16 store of the activated product
-    _GROUPED_RELU2 = 4      # (grouped products only) a bfloat16 store of max(z, 0)^2
+    _RELU2 = 4              # (tcgen05 products only) a bfloat16 store of max(z, 0)^2
     _GATED = 32             # + the activation's code: as _SWIGLU with that gate
 
     def _skinny(self, a, w, fused=False) -> bool:
@@ -295,12 +295,13 @@ class CudaOps:
 
     def _tcgen05(self, a, w, epilogue=0) -> bool:
         """Whether a[M, K] @ w[N, K]^T goes to the tcgen05 kernel. It needs 16-byte aligned
-        rows and at least 128 rows (its tiles are 128 x 256, or 128 x 192 where that takes no more
-        rounds over the SMs, and each persistent block walks whole tiles), and it is chosen where it is faster than the library's product plus the
-        kernel that the library's product then needs: with the fused SwiGLU epilogue, which
-        saves a pass over the widest activation (2048 rows: 100 us against 153 us; 512 rows: 35
-        against 41), when tiles of 128 x 256 fill the SMs to 60 % (measured with those; the
-        narrower ones only take over where the product is chosen by this rule). Plain products and products added into
+        rows and at least 128 rows (its tiles are 128 x 256, 128 x 192 or, by blocks in pairs, 256 x 256, and
+        each persistent block or pair walks whole tiles), and it is chosen where it is faster than the library's
+        product plus the kernel that the library's product then needs: with the fused SwiGLU epilogue, which
+        saves a pass over the widest activation (2048 rows of 2 x 8,192 columns of 2,048: 95 us against 153 us;
+        512 rows: 35 against 41), when tiles of 128 x 256 fill the SMs to 60 % (measured with those; the others
+        only take over where the product is chosen by this rule), and with the squared relu by the rule
+        below. Plain products and products added into
         the residual stream go to the library, which is faster at every row count measured
         (2048 rows: in_proj 37.7 us against 45.3, qkv 20.7 against 30.8, out_proj 14.8 against
         24.8 with the residual epilogue, w2 47 against 62; 8192 rows: 142 / 73 / 49 / 181 us
@@ -313,11 +314,15 @@ class CudaOps:
         if self.tcgen05_always:
             return True
         if epilogue == self._RELU2:
-            # (blocks in pairs on tiles of 256 x 256 against the library's product and a kernel for the
-            # activation: 2,048 rows 2048 -> 8192 54.6 against 60.0 us, 1024 -> 4096 21.5 against 26.5; 1,300
-            # rows, 72 % of three rounds, 41.1 against 41.8)
-            tiles = -(-a.shape[0] // 256) * -(-w.shape[0] // 256)
-            return tiles / (-(-tiles // (self._sm_count // 2)) * (self._sm_count // 2)) >= 0.7
+            # Blocks in pairs on tiles of 256 x 256 take whole rounds whatever rows their tiles hold, and three
+            # tenths of one to start and end; the library's product with a kernel for the activation goes by the
+            # outputs that there are, at seven tenths of that rate. Us in pairs / by the library, 2048 -> 8192: 300
+            # rows 18.6 / 14.3, 512 18.8 / 17.5, 850 29.0 / 27.4, 1,000 29.7 / 31.3, 1,040 38.8 / 32.6, 1,240 40.5 / 39.1, 1,536
+            # 41.9 / 46.2, 1,800 53.3 / 52.8, 2,048 56.7 / 65.6, 4,096 95.7 / 133.7; 1024 -> 4096: 1,024 13.4 / 13.1, 1,600 18.9 /
+            # 17.1, 2,000 19.1 / 19.5, 2,048 19.2 / 21.0, 4,096 30.5 / 40.1. (Lost: 1536 -> 6144 at 1,400 rows 25.6 / 25.0.)
+            pairs = self._sm_count // 2
+            rounds = -(-(-(-a.shape[0] // 256) * -(-w.shape[0] // 256)) // pairs)
+            return a.shape[0] * w.shape[0] >= (0.7 * rounds + 0.29) * pairs * 256 * 256
         if epilogue != self._SWIGLU:
             return False
         tiles = -(-a.shape[0] // 128) * -(-(w.shape[0] // 2) // 128)
@@ -1162,7 +1167,7 @@ class CudaOps:
         gated = torch.empty((rows, width), dtype=x.dtype, device=self.device)
         clamped = activation == "clamped"
         form = (_c_float(limit),) if clamped else \
-            (_c_int(self._GROUPED_RELU2 if ungated else self._SWIGLU),)
+            (_c_int(self._RELU2 if ungated else self._SWIGLU),)
         self._call("mlxone_gemm_tcgen05_grouped" + ("_clamped" if clamped else ""),
                    _c_void_p(_ptr(sorted_x)), _c_int(hidden),
                    _c_void_p(_ptr(gate_up)), _c_ll(gate_up.shape[0]), _c_ll(hidden), _c_ll(hidden),

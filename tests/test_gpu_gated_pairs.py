@@ -60,3 +60,16 @@ def test_pairs_one_after_the_other(ops, k):
     ops.check_errors()
     assert all(torch.equal(gated[0], one) for one in gated)
     assert all(torch.equal(squared[0], one) for one in squared)
+
+
+@pytest.mark.parametrize("k,n,rows,taken", [(2048, 8192, (300, 512, 800, 850, 1040, 1240), False),
+                                            (2048, 8192, (1024, 1536, 2048, 2560, 4096), True),
+                                            (1024, 4096, (512, 1024, 1600, 1800), False), (1024, 4096, (2048, 3000), True)])
+def test_squared_relu_where_pairs_are_faster(ops, k, n, rows, taken):
+    """Tiles count by the rows that they hold: where the pairs' rounds are mostly padding the library's product and
+    the activation's kernel take the call."""
+    if ops._sm_count != 148:
+        pytest.skip("the lines lie where 148 SMs put them")
+    w = torch.empty(n, k, dtype=torch.bfloat16, device=DEVICE)
+    for m in rows:
+        assert ops._tcgen05(torch.empty(m, k, dtype=torch.bfloat16, device=DEVICE), w, ops._RELU2) == taken, m
