@@ -1932,13 +1932,19 @@ class CudaOps:
         blocks_per_sm = self.lib.mlxone_attention_decode_resident(_c_int(head_dim))
         groups = kv_heads * (-(-(heads // kv_heads) // 8))
         wanted = max(self._sm_count * blocks_per_sm // max(requests * groups, 1), 1)
-        # Three or four parts fill the wave to its last places, which clusters of three do not find and a
-        # merge kernel does not pay for where keys are few: one part less. 64 decode steps with prompts of
-        # 350 tokens, 8 key heads: 24 requests 62.4 -> 60.5 ms (800 tokens 75.5 -> 73.6), 17 requests 48.7 ->
-        # 47.2, 9 requests (16 with fillers) 43.6 -> 43.3; behind 1,500 and 3,000 tokens no better and
-        # up to 1 % worse.
-        if wanted in (3, 4) and context_bound <= 1024:
-            wanted -= 1
+        # Two exceptions where keys are few. Clusters of three that need more than 95 % of the places do not all
+        # find them: two parts. (Attention alone at 1,000 keys in 2 / 3 parts, 8 key heads of 64: 22 and 23 requests,
+        # 89 and 93 % of the places, 13.3 / 11.3 and 13.4 / 11.9 us; 24, 97 %, 13.4 / 19.2. Likewise 11 and 12 requests with 8 key heads
+        # of 128, 46 and 48 with 4 of 64, 160 and 168 with 2 of 32. Whole steps of LFM2-700M, 24 requests of 150 to
+        # 1,200 keys: 2 parts 26 us faster of 730; of 3,000: 32 us slower.) And three parts, which a cluster merges,
+        # instead of four with a kernel for the merge: whole steps of 16 requests, LFM2-700M and 350M, 350 and 800 keys
+        # 605 / 610, 615 / 621, 437 / 447, 451 / 461 us. With heads of 128 the longer parts cost what the kernel does
+        # (attention alone at 1,000 keys 14.0 / 10.6 us).
+        if context_bound <= 1024:
+            if wanted == 3 and 3 * requests * groups > 0.95 * self._sm_count * blocks_per_sm:
+                wanted = 2
+            elif wanted == 4 and head_dim <= 64:
+                wanted = 3
         return max(min(wanted, tiles // 4), 1)
 
     def argmax(self, logits):

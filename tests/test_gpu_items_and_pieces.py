@@ -66,3 +66,13 @@ def test_prefill_on_both_sides_of_the_line(ops, plain, portions, histories, wind
     windows; two requests."""
     attention_case(ops, plain, torch.bfloat16, 16, 8, 64, 16, portions=portions, histories=histories,
                    window=window, tensor_cores=True, tcgen05=True)
+
+
+def test_parts_where_clusters_of_three_find_no_place(ops):
+    if ops._sm_count != 148:
+        pytest.skip("the lines lie where 148 SMs put them")
+    for heads, kv_heads, dim, requests, parts in (
+            (24, 8, 64, 23, 3), (24, 8, 64, 24, 2), (32, 8, 128, 11, 3), (32, 8, 128, 12, 2), (16, 4, 64, 46, 3),
+            (16, 4, 64, 48, 2), (8, 2, 32, 160, 3), (8, 2, 32, 168, 2), (24, 8, 64, 16, 3), (32, 8, 128, 9, 4)):
+        assert ops.decode_splits(requests, heads, kv_heads, dim, 1024, None) == parts, (heads, kv_heads, dim, requests)
+    assert ops.decode_splits(24, 24, 8, 64, 2048, None) == 3
