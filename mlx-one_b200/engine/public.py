@@ -119,7 +119,7 @@ class Engine:
                  tokenizer_source: str | Path | None = None,
                  trace_sink: Any = None) -> None:
         """``model``: a model folder (config.json + safetensors) or a loaded model.
-        ``execution_dtype``: "bfloat16" (default) or "float32" (everything in true 32-bit).
+        ``execution_dtype``: "bfloat16" (default) or "float32" (values and sums in 32 bits everywhere).
         ``revision``, ``offline``, ``cache_dir``: the reference's names for fetching a model by
         its hub id (src/mlx_one/engine/public.py:64-85). This engine loads local folders only:
         they are accepted for a local folder (a revision must then be None) and a name that is

@@ -1874,7 +1874,7 @@ class CudaOps:
                                   device=self.device)
         keys = self.lib.mlxone_attention_tcgen05_keys(
             _c_int(tokens - singles), _c_int(rest), _c_int(heads), _c_int(kv_heads), _c_int(ctx.max_context),
-            _c_int(reach or 0), _c_int(splits))
+            _c_int(min(reach or 0, 1 << 30)), _c_int(splits))
         self._call("mlxone_attention_prefill_tcgen05_shaped", *common, _c_int(splits),
                    _c_void_p(_ptr(partial)), _c_int(keys), _c_void_p(_ptr(self.error_flag)))
         if partial is not None:
